@@ -268,6 +268,31 @@ def test_paged_prefill_tensor_core_kernel(hq, hkv, lens):
         expect_close(got.float(), old.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("lens", [[(1, 0), (63, 0), (64, 1), (65, 63)], [(127, 0), (128, 64), (129, 191)], [(3, 4000), (260, 0)]])
+def test_paged_prefill_page_edges(hd, lens):
+    """The tcgen05 prefill kernels at the edges of pages and query blocks, with scores that grow along the keys, so that a row's
+    reference moves again and again.  Probabilities are bf16 on both sides of P V: 2 * 2^-9 of a result of size one."""
+    torch.manual_seed(9)
+    hq, hkv, page = 8, 2, 64
+    q_lens, seq_lens = [a for a, _ in lens], [a + c for a, c in lens]
+    kc, vc, bt = _make_paged(len(lens), seq_lens, hkv, hd, page)
+    for i, n in enumerate(seq_lens):                # key t of a sequence is (1 + t / 40) times as large along one direction
+        t = torch.arange(n, device=DEV)
+        kc[bt[i, t // page].long(), t % page, :, 0] += (1 + t / 40.0).to(torch.bfloat16)[:, None]
+    qs = [0]
+    for n in q_lens:
+        qs.append(qs[-1] + n)
+    q = _randn(qs[-1], hq, hd)
+    q[:, :, 0] = 4.0
+    sl = torch.tensor(seq_lens, dtype=torch.int32, device=DEV)
+    qst = torch.tensor(qs, dtype=torch.int32, device=DEV)
+    for window in (0, 1, 64, 100):
+        got = ops.paged_prefill(q, kc, vc, bt, sl, qst, window=window, impl="tc")
+        want = ref.paged_attention(q, kc, vc, bt, seq_lens, qs, window=window)
+        expect_close(got.float(), want.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
+
+
 @pytest.mark.parametrize("layout,rot", [(0, None), (1, None), (0, 32), (2, 32)])
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_rope_kvwrite(layout, rot, qk_norm):

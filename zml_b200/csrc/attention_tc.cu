@@ -1,4 +1,5 @@
-// Paged prefill attention on the 5th-generation tensor cores (tcgen05 / TMEM / TMA) for sm_100a.
+// Paged prefill attention with the extensions of ZbAttnExt on the 5th-generation tensor cores (tcgen05 / TMEM / TMA) for
+// sm_100a, and the entry point of both tcgen05 prefill kernels (attention_prefill.cu has the one without extensions).
 //
 // Replaces the FA2 / Triton unified-attention prefill path of the reference
 // (zml/attention/flashattn.zig:764-897, zml/attention/triton_attention.zig:140-494) for the common
@@ -18,7 +19,7 @@
 // P = exp2(S - m) as bf16 straight back into tensor memory -> O += P V (A = P from tensor memory,
 // B = V from shared memory in its natural [key][head_dim] layout, i.e. MN-major).
 // Tensor memory columns: S_A 0-63 | S_B 64-127 | P_A 128-159 | P_B 160-191 | O_A 192-319 | O_B 320-447.
-// Three instantiations: kPlain; with what ZbAttnExt adds (kExt); and that with a score cap c of at most kMaxCap (kCapped),
+// Two instantiations: with what ZbAttnExt adds (kExt); and that with a score cap c of at most kMaxCap (kCapped),
 // where the running maximum goes: every score lies in [-c, c], so P = exp2(S') needs no reference and O no rescaling.  Kept
 // first keys join the window's tiles as one list, a chunk is a window whose start is the same for all its positions, a sink
 // is one more term of the sum, and the output gate is applied as the rows are stored.
@@ -30,12 +31,17 @@
 // Every wait is bounded; a wait that runs out records a status and the CTA leaves through its normal exit.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "attention_tiles.cuh"
 #include "common.cuh"
 #include "host_api.h"
 
 int zb_make_tmap_bf16_2d(CUtensorMap* out, const void* base, int rows, int k, int ld, int box_rows);
 int zb_make_tmap_kv_cache(CUtensorMap* out, const void* base, long long slots, int kv_heads, int head_dim, int box_rows);
+int zb_prefill_plain(const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* block_table, const int32_t* seq_lens,
+                     const int32_t* q_start, int batch, int q_blocks, int total_tokens, int num_q_heads, int num_kv_heads, int head_dim,
+                     int max_pages, long long q_stride, float scale, int window, ZbStatus* status, void* stream);
 
 namespace {
 
@@ -53,7 +59,7 @@ constexpr float kMaxCap = 60.f;                    // exp(cap) times the number 
 constexpr float kPolyMax = 0.6f;
 __device__ constexpr float kTanh[6] = {1.0f, -0.333332837f, 0.1333168f, -0.0537679829f, 0.0207513496f, -0.00584964408f};
 constexpr uint32_t kColS = 0, kColP = 128, kColO = 192;
-enum Mode { kPlain, kCapped, kExt };
+enum Mode { kCapped, kExt };
 
 struct PrefillTcParams {
   __nv_bfloat16* out;           // [tokens, num_q_heads, 128]
@@ -69,7 +75,7 @@ struct PrefillTcParams {
   uint32_t v_lbo;               // byte offsets of the MN-major descriptor of V (between 64-column groups / 8-key groups)
   uint32_t v_sbo;
   ZbStatus* status;
-  // not kPlain (ZbAttnExt)
+  // ZbAttnExt
   int keep;
   int chunk;
   float cap_log2;               // cap * log2(e)
@@ -89,11 +95,8 @@ struct PrefillTcParams {
 };
 
 // First key in a position's window or chunk.
-template <bool EXT>
 ZB_DEVICE int first_key_of(const PrefillTcParams& p, int pos) {
-  if constexpr (EXT) {
-    if (p.chunk > 0) return pos / p.chunk * p.chunk;
-  }
+  if (p.chunk > 0) return pos / p.chunk * p.chunk;
   return p.window > 0 ? max(0, pos - p.window + 1) : 0;
 }
 
@@ -175,7 +178,6 @@ template <Mode MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                            const __grid_constant__ CUtensorMap tmap_v, const PrefillTcParams p) {
-  constexpr bool EXT = MODE != kPlain;
   const bool pair = MODE == kExt && p.pair != 0;
   __shared__ float pair_x[4][kQRows];                // differential heads: 1 / row sum of either map, partial sums of squares
   zb_pdl_launch();
@@ -226,9 +228,9 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   const int tok_base = p.q_start[seq] + row_base;
   const int rows_valid = min(kQRows, q_len - row_base);
   const int last_key = min(len, ctx + row_base + kQRows);     // exclusive
-  const int first_key = first_key_of<EXT>(p, ctx + row_base);
-  const int pooled = EXT && p.pool > 0 ? zb_pooled_visible(last_key - 1, p.window, p.pool) : 0;
-  const ZbTileList tiles = zb_visible_tiles(first_key, EXT ? p.keep : 0, (last_key + kKeys - 1) / kKeys, kKeys, pooled);
+  const int first_key = first_key_of(p, ctx + row_base);
+  const int pooled = p.pool > 0 ? zb_pooled_visible(last_key - 1, p.window, p.pool) : 0;
+  const ZbTileList tiles = zb_visible_tiles(first_key, p.keep, (last_key + kKeys - 1) / kKeys, kKeys, pooled);
   const int n_tiles = tiles.count;
 
   if (threadIdx.x == 0) {
@@ -271,24 +273,22 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
             zb_tma_load_2d(q_s + w * kQBytes + c * (kQRows * 128), &tmap_q, q_full, (head0 + w) * kHD + c * 64, tok_base);
     }
     bool ok = true;
-    if constexpr (EXT) {
-      __syncwarp();
-      for (int j = 0; j < tiles.pooled; ++j) {             // the whole warp
-        if (j >= kStages) ok = zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) {
-          *abort_where = 1u;
-          break;
-        }
-        gather_pooled_tile(p, bt, tiles.at(j), pooled, kvh, k_s + stage * kKvBytes, v_s + stage * kKvBytes);
-        if (lane == 0) {
-          zb_mbar_arrive(&k_full[stage]);
-          zb_mbar_arrive(&v_full[stage]);
-        }
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
+    __syncwarp();
+    for (int j = 0; j < tiles.pooled; ++j) {               // the whole warp
+      if (j >= kStages) ok = zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        *abort_where = 1u;
+        break;
+      }
+      gather_pooled_tile(p, bt, tiles.at(j), pooled, kvh, k_s + stage * kKvBytes, v_s + stage * kKvBytes);
+      if (lane == 0) {
+        zb_mbar_arrive(&k_full[stage]);
+        zb_mbar_arrive(&v_full[stage]);
+      }
+      if (++stage == kStages) {
+        stage = 0;
+        phase ^= 1u;
       }
     }
     if (lane == 0 && ok) {
@@ -395,11 +395,11 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     const uint32_t t_s = tmem_base + kColS + w * kKeys + lane_off;
     const uint32_t t_p = tmem_base + kColP + w * 32 + lane_off;
     const uint32_t t_o = tmem_base + kColO + w * kHD + lane_off;
-    float m = MODE == kExt && p.sink ? 0.f : -INFINITY, l = EXT && p.sink ? 1.f : 0.f;
-    const int from = first_key_of<EXT>(p, qpos), from_last = first_key_of<EXT>(p, ctx + row_base + kQRows - 1);
+    float m = MODE == kExt && p.sink ? 0.f : -INFINITY, l = p.sink ? 1.f : 0.f;
+    const int from = first_key_of(p, qpos), from_last = first_key_of(p, ctx + row_base + kQRows - 1);
     // pooled blocks that this row sees, and those that every row of the block sees
-    const int pool_end = EXT && p.pool > 0 ? min(pooled, zb_pooled_visible(qpos, p.window, p.pool)) : 0;
-    const int pool_first = EXT && p.pool > 0 ? zb_pooled_visible(ctx + row_base, p.window, p.pool) : 0;
+    const int pool_end = p.pool > 0 ? min(pooled, zb_pooled_visible(qpos, p.window, p.pool)) : 0;
+    const int pool_first = p.pool > 0 ? zb_pooled_visible(ctx + row_base, p.window, p.pool) : 0;
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
       const uint32_t jj = static_cast<uint32_t>(j);
@@ -418,12 +418,10 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       // predicate per score: predicated-off instructions still take issue slots, and this loop is issue-bound)
       bool full = (key0 + kKeys - 1 <= ctx + row_base) && (key0 + kKeys <= len) && key0 >= from_last;
       int lo = from, hi = min(qpos + 1, len);              // visible: lo <= key < hi, and the kept ones in front
-      if constexpr (EXT) {
-        if (tiles.is_pooled(j)) {
-          full = key0 + kKeys <= pool_first;
-          lo = 0;
-          hi = pool_end;
-        }
+      if (tiles.is_pooled(j)) {
+        full = key0 + kKeys <= pool_first;
+        lo = 0;
+        hi = pool_end;
       }
       uint32_t pw[32];
       float sum0 = 0.f, sum1 = 0.f;
@@ -477,7 +475,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const int kidx = key0 + i;
-            const bool vis = kidx < hi && (kidx >= lo || (EXT && kidx < p.keep));
+            const bool vis = kidx < hi && (kidx >= lo || kidx < p.keep);
             if (!vis) sr[i] = 0xff800000u;             // -inf
             mx_raw = fmaxf(mx_raw, __uint_as_float(sr[i]));
           }
@@ -576,37 +574,20 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       const uint32_t last = static_cast<uint32_t>(n_tiles - 1);
       if (zb_mbar_wait(&o_ready[w], last & 1u, abort_flag)) {
         zb_tc_fence_after();
-        float inv = l > 0.f ? 1.f / l : 0.f;
-        if constexpr (EXT) inv *= p.out_scale;
-        __nv_bfloat16* orow = p.out + (static_cast<size_t>(tok_base + r) * p.num_q_heads + head0 + w) * kHD;
+        const float inv = (l > 0.f ? 1.f / l : 0.f) * p.out_scale;
 #pragma unroll 1
         for (int c0 = 0; c0 < kHD; c0 += 32) {
           uint32_t o[32];
           zb_tmem_ld32(t_o + c0, o);
           zb_tmem_ld_wait();
           if (r < rows_valid) {
-            if constexpr (EXT) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) store_ext8(p, tok_base + r, head0 + w, c0 + 8 * i, o + 8 * i, inv);
-              continue;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t wd[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                wd[q] = zb_pack_bf16x2(__uint_as_float(o[8 * i + 2 * q]) * inv, __uint_as_float(o[8 * i + 2 * q + 1]) * inv);
-              *reinterpret_cast<uint4*>(orow + c0 + 8 * i) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-            }
+            for (int i = 0; i < 4; ++i) store_ext8(p, tok_base + r, head0 + w, c0 + 8 * i, o + 8 * i, inv);
           }
         }
       } else {
         *abort_where = 14u + w;
       }
-    } else if (!EXT && ok && r < rows_valid) {
-      // no key at all (cannot happen for a causal prefill, kept for completeness): zeros
-      __nv_bfloat16* orow = p.out + (static_cast<size_t>(tok_base + r) * p.num_q_heads + head0 + w) * kHD;
-      for (int c = 0; c < kHD; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
 
@@ -632,10 +613,10 @@ constexpr int kSmemBytes = 2 * kQBytes + 2 * kStages * kKvBytes + 1024 + 256;
 
 extern "C" {
 
-// 1 when the tensor-core prefill kernel takes this shape (head_dim 128, 64-token pages, an even number of query
-// heads per KV head), else 0: the caller then uses the mma.sync kernel.
+// 1 when a tensor-core prefill kernel takes this shape (head_dim 128, without ZbAttnExt also 64; 64-token pages, an even number of
+// query heads per KV head), else 0: the caller then uses the mma.sync kernel.
 int zb_paged_prefill_tc_supported(int num_q_heads, int num_kv_heads, int head_dim, int page_size) {
-  if (head_dim != kHD || page_size != kKeys || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
+  if ((head_dim != kHD && head_dim != 64) || page_size != kKeys || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
   return ((num_q_heads / num_kv_heads) % 2) == 0 ? 1 : 0;
 }
 
@@ -646,21 +627,25 @@ int zb_paged_prefill_tc_ext_supported(float cap, int pair) { return cap == 0.f |
 // `v_lbo` / `v_sbo` = 0 select the defaults of the V descriptor (8192 / 1024 bytes).
 int zb_paged_prefill_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* block_table,
                         const int32_t* seq_lens, const int32_t* q_start, int batch, int total_q_blocks128, int total_tokens,
-                        int num_q_heads, int num_kv_heads, int max_pages, long long q_stride, float scale, int window,
+                        int num_q_heads, int num_kv_heads, int head_dim, int max_pages, long long q_stride, float scale, int window,
                         unsigned v_lbo, unsigned v_sbo, const ZbAttnExt* ext, void* stream) {
   if (batch <= 0 || total_q_blocks128 <= 0) return 0;
-  if (!zb_paged_prefill_tc_supported(num_q_heads, num_kv_heads, kHD, kKeys)) return -32;
+  if (!zb_paged_prefill_tc_supported(num_q_heads, num_kv_heads, head_dim, kKeys) || (ext != nullptr && head_dim != kHD)) return -32;
   ZbDeviceState* st = zb_device_state();
   if (!st) return -20;
-  if (ext != nullptr && (!zb_paged_prefill_tc_ext_supported(ext->cap, ext->pair) || ext->out_f32 != 0 || (ext->pair != 0 && ext->gate != nullptr)))
+  total_q_blocks128 = std::min(total_q_blocks128, total_tokens / kQRows + batch);      // a caller may count blocks of 64 rows
+  if (ext == nullptr)
+    return zb_prefill_plain(q, k_cache, v_cache, out, block_table, seq_lens, q_start, batch, total_q_blocks128, total_tokens, num_q_heads,
+                            num_kv_heads, head_dim, max_pages, q_stride, scale, window, st->status, stream);
+  if ((!zb_paged_prefill_tc_ext_supported(ext->cap, ext->pair) || ext->out_f32 != 0 || (ext->pair != 0 && ext->gate != nullptr)))
     return -34;
-  if (ext != nullptr && ext->pair != 0 && (ext->ldo != 0 || ext->scaled)) return -34;
-  if (ext != nullptr && ext->pool != 0 &&
+  if (ext->pair != 0 && (ext->ldo != 0 || ext->scaled)) return -34;
+  if (ext->pool != 0 &&
       (ext->pool < 0 || window <= 0 || ext->chunk != 0 || ext->pool_rows <= 0 || ext->pool_k == nullptr || ext->pool_v == nullptr))
     return -34;
-  static bool configured[3][16] = {};
-  const Mode mode = ext == nullptr ? kPlain : (ext->cap > 0.f ? kCapped : kExt);
-  const auto kernel = mode == kPlain ? zb_paged_prefill_tc_kernel<kPlain> : (mode == kCapped ? zb_paged_prefill_tc_kernel<kCapped> : zb_paged_prefill_tc_kernel<kExt>);
+  static bool configured[2][16] = {};
+  const Mode mode = ext->cap > 0.f ? kCapped : kExt;
+  const auto kernel = mode == kCapped ? zb_paged_prefill_tc_kernel<kCapped> : zb_paged_prefill_tc_kernel<kExt>;
   if (const int rc = zb_config_smem_once(kernel, kSmemBytes, configured[mode])) return rc;
   CUtensorMap tq, tk, tv;
   // q as a [tokens, heads * 128] matrix with leading dimension q_stride: boxes of 128 rows x 64 columns
@@ -685,29 +670,27 @@ int zb_paged_prefill_tc(const void* q, const void* k_cache, const void* v_cache,
   p.v_lbo = v_lbo ? v_lbo : 8192u;
   p.v_sbo = v_sbo ? v_sbo : 1024u;
   p.status = st->status;
-  if (ext != nullptr) {
-    p.keep = ext->keep;
-    p.chunk = ext->chunk;
-    if (ext->cap > 0.f) {
-      p.cap_log2 = ext->cap * 1.4426950408889634f;
-      p.cap_in = 2.f * scale * 1.4426950408889634f / ext->cap;
-      p.cap_x = scale / ext->cap;
-    }
-    p.pair = ext->pair;
-    p.pair_lambda = ext->pair_lambda;
-    p.pair_scale = ext->pair_scale;
-    p.pair_eps = ext->pair_eps;
-    p.sink = ext->sink;
-    p.vdim = ext->vdim;
-    p.gate = reinterpret_cast<const __nv_bfloat16*>(ext->gate);
-    p.ldg = ext->ldg;
-    p.pool = ext->pool;
-    p.pool_rows = ext->pool_rows;
-    p.pool_k = reinterpret_cast<const __nv_bfloat16*>(ext->pool_k);
-    p.pool_v = reinterpret_cast<const __nv_bfloat16*>(ext->pool_v);
-    p.ldo = ext->ldo > 0 ? ext->ldo : static_cast<long long>(num_q_heads) * ext->vdim;
-    p.out_scale = ext->scaled ? ext->out_scale : 1.f;
+  p.keep = ext->keep;
+  p.chunk = ext->chunk;
+  if (ext->cap > 0.f) {
+    p.cap_log2 = ext->cap * 1.4426950408889634f;
+    p.cap_in = 2.f * scale * 1.4426950408889634f / ext->cap;
+    p.cap_x = scale / ext->cap;
   }
+  p.pair = ext->pair;
+  p.pair_lambda = ext->pair_lambda;
+  p.pair_scale = ext->pair_scale;
+  p.pair_eps = ext->pair_eps;
+  p.sink = ext->sink;
+  p.vdim = ext->vdim;
+  p.gate = reinterpret_cast<const __nv_bfloat16*>(ext->gate);
+  p.ldg = ext->ldg;
+  p.pool = ext->pool;
+  p.pool_rows = ext->pool_rows;
+  p.pool_k = reinterpret_cast<const __nv_bfloat16*>(ext->pool_k);
+  p.pool_v = reinterpret_cast<const __nv_bfloat16*>(ext->pool_v);
+  p.ldo = ext->ldo > 0 ? ext->ldo : static_cast<long long>(num_q_heads) * ext->vdim;
+  p.out_scale = ext->scaled ? ext->out_scale : 1.f;
   const cudaError_t le = zb_launch(kernel, dim3(total_q_blocks128, num_q_heads / 2), dim3(kThreads), kSmemBytes,
                                    reinterpret_cast<cudaStream_t>(stream), tq, tk, tv, p);
   zb_count_launch(1);

@@ -389,7 +389,7 @@ def _ext(ext):
     return None if ext is None else C.addressof(ext)
 
 
-# ZB_ATTN_TC=0: prefill attention always on the mma.sync kernel (the tensor-core kernel takes head_dim 128,
+# ZB_ATTN_TC=0: prefill attention always on the mma.sync kernel (the tensor-core kernels take head_dim 64 and 128,
 # 64-token pages and an even number of query heads per KV head)
 import os as _os
 _ATTN_TC = _os.environ.get("ZB_ATTN_TC", "1") != "0"
@@ -398,7 +398,9 @@ _ATTN_TC = _os.environ.get("ZB_ATTN_TC", "1") != "0"
 def _tc_takes(q, k_cache, ext) -> bool:
     l = _lib.lib()
     ok = bool(l.zb_paged_prefill_tc_supported(q.shape[1], k_cache.shape[2], q.shape[2], k_cache.shape[1])) and q.stride(0) % 8 == 0
-    return ok and (ext is None or bool(l.zb_paged_prefill_tc_ext_supported(ext.cap, ext.pair)))
+    if q.shape[2] == 64 and ext is None:            # tensor maps start on 16 bytes; the mma.sync kernel takes other pointers
+        return ok and (q.data_ptr() | k_cache.data_ptr()) % 16 == 0
+    return ok and (ext is None or (q.shape[2] == 128 and bool(l.zb_paged_prefill_tc_ext_supported(ext.cap, ext.pair))))
 
 
 def prefill_on_tc(q, k_cache, ext=None) -> bool:
@@ -434,7 +436,7 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
     if tc_ok and (impl == "tc" or (impl == "auto" and _ATTN_TC)):
         rc = l.zb_paged_prefill_tc(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _ptr(seq_lens), _ptr(q_start), b, nqb, t,
-            hq, hkv, block_table.shape[1], q.stride(0), float(scale if scale is not None else 1.0 / math.sqrt(hd)), int(window),
+            hq, hkv, hd, block_table.shape[1], q.stride(0), float(scale if scale is not None else 1.0 / math.sqrt(hd)), int(window),
             int(_os.environ.get("ZB_ATTN_V_LBO", "0")), int(_os.environ.get("ZB_ATTN_V_SBO", "0")), _ext(ext), _lib.stream_ptr())
         _lib.check(rc, "zb_paged_prefill_tc")
         return out
