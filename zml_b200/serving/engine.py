@@ -20,9 +20,11 @@ from __future__ import annotations
 
 import contextlib
 import time
+from array import array
 from dataclasses import dataclass, field
 from typing import Optional, Sequence as Seq
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -124,10 +126,10 @@ class Engine:
         i32 = dict(dtype=torch.int32, device=self.device)
         mb = max_batch
         # static decode buffers (graph inputs / outputs)
-        self.d_ids = torch.zeros(mb, **i32)
-        self.d_pos = torch.zeros(mb, **i32)
-        self.d_seq = torch.zeros(mb, **i32)
-        self.d_slot = torch.full((mb,), -1, **i32)
+        # token, position, length, cache slot and state slot of every row: rows of one tensor, so that they go up in one copy
+        self.d_rows = torch.zeros((5, mb), **i32)
+        self.d_ids, self.d_pos, self.d_seq, self.d_slot, self.d_sslot = self.d_rows.unbind(0)
+        self.d_slot.fill_(-1)
         self.d_bt = torch.zeros((mb, self.max_pages), **i32)
         self.d_hist = torch.zeros((history_steps, mb), **i32)
         self.d_step = torch.zeros(1, **i32)
@@ -139,7 +141,7 @@ class Engine:
         self.num_slots = num_state_slots if num_state_slots is not None else 2 * mb
         self.scratch_slot = self.num_slots
         self.slot_free = list(range(self.num_slots - 1, -1, -1))
-        self.d_sslot = torch.full((mb,), self.scratch_slot, **i32)
+        self.d_sslot.fill_(self.scratch_slot)
         self.d_qs = torch.arange(mb + 1, **i32)
         self.stateful = hasattr(model, "alloc_state")
         if self.stateful:
@@ -153,6 +155,20 @@ class Engine:
         """Seed of the sampler for what follows; restarts its draw counter."""
         self.seed = int(seed)
         self.d_rng.copy_(torch.tensor([self.seed, 0], dtype=torch.int64))
+
+    def _host(self, *shape) -> torch.Tensor:
+        """An int32 tensor for a copy to the device."""
+        return torch.empty(shape, dtype=torch.int32, pin_memory=self.on_gpu)
+
+    def _tables(self, out: np.ndarray, requests) -> None:
+        """Block tables of `requests` into the rows of `out` (zeros behind their pages and in further rows)."""
+        n, width = len(requests), out.shape[1]
+        flat = array("i")
+        for r in requests:
+            flat.extend(r.pages)
+            flat.frombytes(bytes(4 * (width - len(r.pages))))
+        out[:n] = np.frombuffer(flat, dtype=np.int32).reshape(n, width)
+        out[n:] = 0
 
     def _pin(self, t: torch.Tensor) -> torch.Tensor:
         return t.pin_memory() if self.on_gpu else t
@@ -232,21 +248,22 @@ class Engine:
     def _varlen_meta(self, chunk, rows: list[int], stats: Optional[GenerationStats]):
         """(token ids, AttnMeta) on the device of one flattened varlen batch of (request, start, end) token ranges;
         `rows`: the rows of the batch whose logits are needed."""
-        ps = self.page_size
-        ids, pos, slots, qs, sl = [], [], [], [0], []
-        bt = torch.zeros((len(chunk), self.max_pages), dtype=torch.int32)
-        for i, (r, a, b) in enumerate(chunk):
-            ids.extend(r.prompt[a:b])
-            pos.extend(range(a, b))
-            pg = r.pages
-            slots.extend(pg[p // ps] * ps + p % ps for p in range(a, b))
-            qs.append(qs[-1] + (b - a))
+        ps, total = self.page_size, sum(b - a for _, a, b in chunk)
+        host, bt_h = self._host(3, total), self._host(len(chunk), self.max_pages)
+        ids, pos, slots = host.numpy()
+        qs, sl = [0], []
+        for r, a, b in chunk:
+            at = slice(qs[-1], qs[-1] + (b - a))
+            ids[at] = array("i", r.prompt[a:b])
+            pos[at] = np.arange(a, b, dtype=np.int32)
+            pg = np.array(r.pages[a // ps:(b - 1) // ps + 1], dtype=np.int32)
+            slots[at] = pg[pos[at] // ps - a // ps] * ps + pos[at] % ps
+            qs.append(at.stop)
             sl.append(b)
-            bt[i, :len(pg)] = torch.tensor(pg, dtype=torch.int32)
-        host = self._pin(torch.tensor([ids, pos, slots], dtype=torch.int32))
+        self._tables(bt_h.numpy(), [r for r, _, _ in chunk])
         sslots = [max(r.slot, 0) if self.stateful else 0 for r, _, _ in chunk]
-        meta_h = self._pin(torch.tensor(qs + sl + sslots + rows, dtype=torch.int32))
-        bt_h = self._pin(bt)
+        meta_h = self._host(len(qs) + len(sl) + len(sslots) + len(rows))
+        meta_h.numpy()[:] = array("i", qs + sl + sslots + rows)
         dev = self._to_dev(host, stats)
         meta_d = self._to_dev(meta_h, stats)
         bt_d = self._to_dev(bt_h, stats)
@@ -293,7 +310,14 @@ class Engine:
         if all(b - a == 1 and a > 0 for _, a, b in chunk) and len(chunk) <= self.max_batch:
             lg = self._step_decode(chunk)
             rows = [i for i, w in enumerate(want) for _ in w]
-            lg = lg[torch.tensor(rows, device=lg.device)] if rows else None
+            if rows == list(range(lg.shape[0])):
+                lg = lg.clone()                  # the capture's buffer is written again by the next step
+            elif rows:
+                at = self._host(len(rows))
+                at.numpy()[:] = array("i", rows)
+                lg = lg.index_select(0, self._to_dev(at))
+            else:
+                lg = None
         else:
             rows, base = [], 0
             for (r, a, b), w in zip(chunk, want):
@@ -312,15 +336,15 @@ class Engine:
     def _step_decode(self, chunk) -> torch.Tensor:
         b, ps = len(chunk), self.page_size
         bb = min(_bucket(b) if self.use_graphs else b, self.max_batch)
-        st = torch.zeros((5, bb), dtype=torch.int32)
-        st[3] = -1
-        st[4] = self.scratch_slot
-        bt = torch.zeros((bb, self.max_pages), dtype=torch.int32)
-        for i, (r, a, _) in enumerate(chunk):
-            st[:4, i] = torch.tensor([r.prompt[a], a, a + 1, r.pages[a // ps] * ps + a % ps], dtype=torch.int32)
-            if self.stateful:
-                st[4, i] = r.slot
-            bt[i, :len(r.pages)] = torch.tensor(r.pages, dtype=torch.int32)
+        st, bt = self._host(5, bb), self._host(bb, self.max_pages)
+        rows = st.numpy()
+        rows[0, :b] = array("i", [r.prompt[a] for r, a, _ in chunk])
+        rows[1, :b] = array("i", [a for _, a, _ in chunk])
+        rows[2, :b] = rows[1, :b] + 1
+        rows[3, :b] = array("i", [r.pages[a // ps] * ps + a % ps for r, a, _ in chunk])
+        rows[4, :b] = array("i", [r.slot for r, _, _ in chunk]) if self.stateful else self.scratch_slot
+        rows[:3, b:], rows[3, b:], rows[4, b:] = 0, -1, self.scratch_slot
+        self._tables(bt.numpy(), [r for r, _, _ in chunk])
         self._upload_decode(bb, st, bt, None)
         self.d_step.zero_()
         max_total = self.max_pages * ps
@@ -332,11 +356,14 @@ class Engine:
     def _upload_decode(self, bb: int, st: torch.Tensor, bt: torch.Tensor, stats: Optional[GenerationStats]) -> None:
         """Device state of the first bb batch rows: st [5, bb] = token, position, length, cache slot (negative: none) and
         state slot; bt [bb, max_pages] block tables."""
-        st_d = self._to_dev(self._pin(st), stats)
-        self.d_ids[:bb].copy_(st_d[0]); self.d_pos[:bb].copy_(st_d[1]); self.d_seq[:bb].copy_(st_d[2]); self.d_slot[:bb].copy_(st_d[3])
-        if self.stateful:
-            self.d_sslot[:bb].copy_(st_d[4])
-        self.d_bt[:bb].copy_(self._to_dev(self._pin(bt), stats))
+        for t in (st, bt):
+            if stats is not None:
+                stats.h2d_bytes += t.numel() * t.element_size()
+        if bb == self.max_batch:
+            self.d_rows.copy_(st if st.is_pinned() else self._pin(st), non_blocking=True)
+        else:
+            self.d_rows[:, :bb].copy_(self._to_dev(st if st.is_pinned() else self._pin(st)))
+        self.d_bt[:bb].copy_(bt if bt.is_pinned() else self._pin(bt), non_blocking=True)
 
     # ------------------------------------------------------------------ decode
     def _decode_body(self, b: int, strategy, num_splits, max_seq_len):
