@@ -79,6 +79,30 @@ def test_gated_delta_scan_chunks_and_decode(hk, hv, dk, dv):
         prior = [p + n for p, n in zip(prior, lens)]
 
 
+@pytest.mark.parametrize("hk,hv,dk,dv,decay", [(2, 4, 128, 128, 1.5), (1, 2, 64, 96, -6.0), (1, 1, 128, 32, 0.0), (2, 2, 64, 256, -2.0)])
+def test_gated_delta_chunks_match_the_walk(hk, hv, dk, dv, decay, monkeypatch):
+    """The chunked kernels against the walk token by token (both fp32 inside): chunk edges, an empty sequence, a continued one, strong
+    and weak decays.  Outputs are bf16 on both sides; a state element is a sum over at most 65 tokens of terms below one."""
+    torch.manual_seed(dk + dv)
+    lens, prior = [16, 0, 65, 17], [0, 4, 9, 0]
+    qs, sl, slots = (v.to(DEV) for v in _seq_meta(lens, prior))
+    t, val = sum(lens), hv * dv
+    proj = torch.randn(t, 2 * hk * dk + 2 * val + (2 * hv + 7) // 8 * 8, device=DEV).bfloat16()
+    o = 2 * hk * dk + val
+    a_log, dtb, nw = decay + 0.5 * torch.randn(hv, device=DEV), torch.randn(hv, device=DEV), torch.ones(dv, device=DEV).bfloat16()
+    start = torch.randn(4, hv, dk, dv, device=DEV) * 0.1
+    res = []
+    for chunks in (True, False):
+        monkeypatch.setattr(la, "_delta_in_chunks", lambda tokens, seqs, c=chunks: c)
+        state = start.clone()
+        out = la.gated_delta_scan(proj[:, :o], proj[:, o:o + val], proj[:, o + val:o + val + hv], proj[:, o + val + hv:o + val + 2 * hv], a_log, dtb, nw, 1e-6,
+                                  state, qs, sl, slots, hk, hv, dk, dv)
+        res.append((out.float(), state))
+    expect_close(res[0][0], res[1][0], atol=1e-2, rtol=1e-2, min_close=0.999)
+    expect_close(res[0][1], res[1][1], atol=2e-5, rtol=1e-5, min_close=1.0)
+    assert torch.equal(res[0][1][0], start[0])               # the empty sequence's slot
+
+
 def test_sigmoid_gate_mul():
     buf = torch.randn(37, 256 + 128, device=DEV).bfloat16()
     x = buf[:, :128].clone()
