@@ -103,6 +103,22 @@ def test_gated_delta_chunks_match_the_walk(hk, hv, dk, dv, decay, monkeypatch):
     assert torch.equal(res[0][1][0], start[0])               # the empty sequence's slot
 
 
+@pytest.mark.parametrize("k,c", [(2, 8), (4, 1032), (5, 64)])
+def test_causal_conv1d_token_blocks(k, c):
+    """Prompts cut along their tokens: block edges, sequences shorter than the taps, a continued and an empty one; the same roundings as
+    the reference, so a bf16 unit in the last place at most, and the cache to the bit."""
+    torch.manual_seed(k)
+    lens, prior = [32, 0, 65, 1], [0, 3, 40, 2]
+    qs, sl, slots = _seq_meta(lens, prior)
+    w, x = (torch.randn(c, k) * 0.5).bfloat16(), torch.randn(sum(lens), c).bfloat16()
+    st_cpu = torch.randn(4, k - 1, c).bfloat16()
+    st_gpu = st_cpu.to(DEV)
+    want = la.causal_conv1d_reference(x, w, st_cpu, qs, sl, slots, silu=True)
+    got = la.causal_conv1d(x.to(DEV), w.to(DEV), st_gpu, qs.to(DEV), sl.to(DEV), slots.to(DEV), silu=True)
+    expect_close(got.float().cpu(), want.float(), atol=1e-2, rtol=1e-2, min_close=1.0)
+    assert torch.equal(st_gpu.cpu(), st_cpu)
+
+
 def test_sigmoid_gate_mul():
     buf = torch.randn(37, 256 + 128, device=DEV).bfloat16()
     x = buf[:, :128].clone()

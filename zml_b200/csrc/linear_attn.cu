@@ -77,6 +77,119 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_kernel(const ConvParams 
   for (int j = 0; j < K - 1; ++j) st[static_cast<size_t>(j) * p.channels] = __float2bfloat16(win[j]);
 }
 
+// The same for rows that start on 16 bytes: a thread has eight channels and walks kConvTokens tokens of one sequence, so a prompt is cut
+// along its tokens as well (8192 channels, 8192 tokens of 7 sequences: the walk of a whole sequence above took 1214 us, bound by
+// the latency of one load per token; TODO).  The inputs in front of a block are read again.  The block at a sequence's start owns
+// its cache: it reads it before it writes the sequence's last inputs to it.
+constexpr int kConvTokens = 32;
+
+ZB_DEVICE void conv_unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = zb_unpack_bf16x2(w[i]);
+    f[2 * i] = v.x;
+    f[2 * i + 1] = v.y;
+  }
+}
+ZB_DEVICE uint4 conv_pack8(const float (&f)[8]) {
+  return make_uint4(zb_pack_bf16x2(f[0], f[1]), zb_pack_bf16x2(f[2], f[3]), zb_pack_bf16x2(f[4], f[5]), zb_pack_bf16x2(f[6], f[7]));
+}
+ZB_DEVICE float conv_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+
+template <int K>
+__global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const ConvParams p, int num_seqs) {
+  zb_pdl_launch();
+  zb_pdl_wait();
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8, cid = blockIdx.y;
+  // Sequence s has the blocks from q_start[s] / kConvTokens + s on, which are no fewer than it needs.
+  int s = 0;
+  for (int hi = num_seqs; hi - s > 1;) {
+    const int mid = (s + hi) >> 1;
+    if (p.q_start[mid] / kConvTokens + mid <= cid) s = mid; else hi = mid;
+  }
+  const int t0 = p.q_start[s], t1 = p.q_start[s + 1], a = t0 + (cid - (t0 / kConvTokens + s)) * kConvTokens, b = min(a + kConvTokens, t1);
+  if (c >= p.channels || a >= t1) return;
+  const bool fresh = p.seq_lens[s] - (t1 - t0) <= 0;
+  if (!ZB_BC_OK(p.slots[s], ZB_BC_STATE_SLOTS, kKernelCausalConv, 2)) return;
+  __nv_bfloat16* st = p.state + static_cast<size_t>(p.slots[s]) * (K - 1) * p.channels + c;
+  auto input = [&](int t, float (&x)[8]) {
+    conv_unpack8(*reinterpret_cast<const uint4*>(p.x + t * p.ldx + c), x);
+    if (p.pre != nullptr) {
+      float g[8];
+      conv_unpack8(*reinterpret_cast<const uint4*>(p.pre + t * p.ldpre + c), g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = conv_round(x[i] * g[i]);
+    }
+  };
+  float w[K][8], win[K - 1][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[j][i] = __bfloat162float(p.w[static_cast<size_t>(c + i) * K + j]);
+#pragma unroll
+  for (int j = 0; j < K - 1; ++j) {                  // the inputs of tokens a - (K - 1) + j
+    const int t = a - (K - 1) + j;
+    if (t >= t0) {
+      input(t, win[j]);
+    } else if (!fresh) {
+      conv_unpack8(*reinterpret_cast<const uint4*>(st + static_cast<size_t>(t - t0 + K - 1) * p.channels), win[j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) win[j][i] = 0.f;
+    }
+  }
+  if (a == t0) {
+    // the sequence's last K - 1 inputs, those in front of its first token among them
+    uint4 last[K - 1];
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) {
+      const int t = t1 - (K - 1) + j;
+      float x[8];
+      if (t >= t0) {
+        input(t, x);
+      } else {
+#pragma unroll
+        for (int q = 0; q < K - 1; ++q)
+          if (q == t - t0 + K - 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = win[q][i];
+          }
+      }
+      last[j] = conv_pack8(x);
+    }
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) *reinterpret_cast<uint4*>(st + static_cast<size_t>(j) * p.channels) = last[j];
+  }
+#pragma unroll 4
+  for (int t = a; t < b; ++t) {
+    float x[8], acc[8];
+    input(t, x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float v = w[K - 1][i] * x[i];
+#pragma unroll
+      for (int j = 0; j < K - 1; ++j) v += w[j][i] * win[j][i];
+      v = conv_round(v);
+      if (p.silu) v = v / (1.f + __expf(-v));
+      acc[i] = v;
+    }
+#pragma unroll
+    for (int j = 0; j + 1 < K - 1; ++j)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) win[j][i] = win[j + 1][i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) win[K - 2][i] = x[i];
+    if (p.post != nullptr) {
+      float g[8];
+      conv_unpack8(*reinterpret_cast<const uint4*>(p.post + t * p.ldpost + c), g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = conv_round(acc[i]) * g[i];
+    }
+    *reinterpret_cast<uint4*>(p.out + t * p.ldo + c) = conv_pack8(acc);
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 struct GdnParams {
   const __nv_bfloat16* mix;    // [T, ld_mix]: q heads | k heads | v heads (after conv + SiLU)
@@ -249,11 +362,11 @@ int launch_gdn(const GdnParams& p, int num_seqs, cudaStream_t s) {
 
 extern "C" {
 
-// Depthwise causal conv over a flattened varlen batch; `kernel_size` taps per channel, 2..5.
+// Depthwise causal conv over a flattened varlen batch of `tokens` rows; `kernel_size` taps per channel, 2..5.
 int zb_causal_conv1d(const void* x, long long ldx, const void* pre, long long ldpre, const void* post,
                      long long ldpost, const void* w, void* out, long long ldo, void* state,
                      const int32_t* q_start, const int32_t* seq_lens, const int32_t* slots, int num_seqs,
-                     int channels, int kernel_size, int silu, void* stream) {
+                     int tokens, int channels, int kernel_size, int silu, void* stream) {
   if (num_seqs <= 0 || channels <= 0) return 0;
   ConvParams p;
   p.x = reinterpret_cast<const __nv_bfloat16*>(x);
@@ -272,6 +385,20 @@ int zb_causal_conv1d(const void* x, long long ldx, const void* pre, long long ld
   p.channels = channels;
   p.silu = silu;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const auto at16 = [](const void* q, long long ld) { return q == nullptr || ((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld & 7) == 0); };
+  if (channels % 8 == 0 && at16(x, ldx) && at16(pre, ldpre) && at16(post, ldpost) && at16(out, ldo) && at16(state, 0) &&
+      tokens / kConvTokens + num_seqs <= 65535) {
+    const dim3 blocks((channels / 8 + 127) / 128, tokens / kConvTokens + num_seqs);
+    switch (kernel_size) {
+      case 2: zb_launch(zb_causal_conv1d_blocks_kernel<2>, blocks, dim3(128), 0, s, p, num_seqs); break;
+      case 3: zb_launch(zb_causal_conv1d_blocks_kernel<3>, blocks, dim3(128), 0, s, p, num_seqs); break;
+      case 4: zb_launch(zb_causal_conv1d_blocks_kernel<4>, blocks, dim3(128), 0, s, p, num_seqs); break;
+      case 5: zb_launch(zb_causal_conv1d_blocks_kernel<5>, blocks, dim3(128), 0, s, p, num_seqs); break;
+      default: return -70;
+    }
+    zb_count_launch(1);
+    return static_cast<int>(cudaGetLastError());
+  }
   const dim3 grid((channels + 127) / 128, num_seqs);
   switch (kernel_size) {
     case 2: zb_launch(zb_causal_conv1d_kernel<2>, grid, dim3(128), 0, s, p); break;

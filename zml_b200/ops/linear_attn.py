@@ -25,7 +25,7 @@ from . import _lib
 
 _p, _i, _ll, _f = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 _lib.register_signature("zb_causal_conv1d", _i, [_p, _ll, _p, _ll, _p, _ll, _p, _p, _ll, _p, _p, _p, _p, _i, _i,
-                                                _i, _i, _p])
+                                                _i, _i, _i, _p])
 _lib.register_signature("zb_gated_delta_scan", _i, [_p, _ll, _p, _ll, _p, _p, _ll, _p, _p, _p, _f, _p, _p, _ll,
                                                    _p, _p, _p, _i, _i, _i, _i, _i, _p])
 _lib.register_signature("zb_gated_delta_rec_bytes", C.c_size_t, [_i, _i, _i])
@@ -82,7 +82,7 @@ def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, si
     rc = _lib.lib().zb_causal_conv1d(
         _ptr(x), x.stride(0), _ptr(pre), pre.stride(0) if pre is not None else 0, _ptr(post),
         post.stride(0) if post is not None else 0, _ptr(w), _ptr(out), out.stride(0), _ptr(state),
-        _ptr(q_start), _ptr(seq_lens), _ptr(slots), seq_lens.shape[0], c, k, 1 if silu else 0, _lib.stream_ptr())
+        _ptr(q_start), _ptr(seq_lens), _ptr(slots), seq_lens.shape[0], t, c, k, 1 if silu else 0, _lib.stream_ptr())
     _lib.check(rc, "zb_causal_conv1d")
     return out
 
