@@ -112,6 +112,29 @@ def test_gemm_emits_row_statistics_of_its_output(m, n, k):
     assert torch.equal(out3, out) and torch.equal(stats3.total(), stats.total())
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (3, 17, 72), (8, 130, 1032), (5, 4800, 2056), (7, 96, 4096)])
+def test_gemm_few_tokens(m, n, k):
+    """The kernel of up to 8 tokens at the edges of its tiles (16 rows, 1024 columns, more tiles than CTAs), all epilogues, against fp32:
+    a bf16 rounding of a result of size one (2^-9), a few of them at size four."""
+    torch.manual_seed(m + n)
+    a, w, bias = _randn(m, k), _randn(n, k, scale=1.0 / math.sqrt(k)), _randn(n)
+    base = a.float() @ w.float().t()
+    expect_close(ops.gemm(a, w, out_dtype=torch.float32, static_w=True), base, atol=1e-4, rtol=1e-4, min_close=1.0)
+    res = torch.randn(m, (n + 7) // 8 * 8, device=DEV).bfloat16()[:, :n]
+    want = torch.relu(base + bias.float() + res.float()).square()
+    got = ops.gemm(a, w, bias=bias, residual=res, act="relu2")
+    expect_close(got.float(), want, atol=2e-2, rtol=2e-2, min_close=1.0)
+    scale = torch.rsqrt(a.float().pow(2).mean(-1, keepdim=True) + 1e-5)
+    inplace = res.clone() if n % 8 == 0 else torch.empty_strided(res.shape, res.stride(), dtype=res.dtype, device=DEV).copy_(res)
+    out, stats = ops.gemm(a, w, residual=inplace, out=inplace, row_stats=ops.row_sumsq(a), emit_stats=True)
+    expect_close(out.float(), base * scale + res.float(), atol=2e-2, rtol=2e-2, min_close=1.0)
+    expect_close(stats.total(), out.float().pow(2).sum(-1), atol=1e-2, rtol=1e-4, min_close=1.0)
+    if n % 2 == 0:
+        act = ops.gemm(a, ops.interleave_gate_up(w), row_stats=ops.row_sumsq(a), swiglu=True)
+        sc = base * scale
+        expect_close(act.float(), torch.nn.functional.silu(sc[:, :n // 2]) * sc[:, n // 2:], atol=2e-2, rtol=2e-2, min_close=1.0)
+
+
 @pytest.mark.parametrize("rows,d", [(1, 2048), (33, 4096), (64, 8192), (5, 1024 + 8), (3, 16384)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm(rows, d, with_res):

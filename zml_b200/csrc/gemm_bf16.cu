@@ -1722,6 +1722,9 @@ size_t zb_gemm_workspace_bytes(int m, int n, int k, int num_sms) {
 
 }  // extern "C"
 
+int zb_gemm_stream_wants(const void* a, const void* w, int m, int n, int k);
+int zb_gemm_stream_launch(const void* a, const void* w, void* out, const void* residual, const void* bias, int m, int n, int k, int lda, int ldw,
+                          int ldo, int out_f32, int static_w, const ZbGemmEpi* epi, int* out_parts, int num_sms, cudaStream_t stream);
 int zb_gemm_2cta_wants(int m, int n, int k);
 int zb_gemm_2cta_launch(const void* a, const void* w, void* out, const void* residual, const void* bias, int m, int n, int k, int lda,
                         int ldw, int ldo, int out_f32, const ZbGemmEpi* epi, ZbStatus* status, int num_sms, cudaStream_t stream);
@@ -1766,6 +1769,8 @@ int gemm_impl(const void* a, const void* w, void* out, const void* residual, con
   if (!out_f32 && (ldo % 8) != 0) return -11;
   int rc = check_epi(epi, m, n, ldo, out_f32, residual, bias);
   if (rc != 0) return rc;
+  if ((band == nullptr || band->mode == 0) && split_hint <= 0 && zb_gemm_stream_wants(a, w, m, n, k))
+    return zb_gemm_stream_launch(a, w, out, residual, bias, m, n, k, lda, ldw, ldo, out_f32, static_w, epi, out_parts, num_sms, stream);
   if ((band == nullptr || band->mode == 0) && split_hint <= 0 && zb_gemm_2cta_wants(m, n, k)) {
     // prefill-sized: 256 x 256 tiles on pairs of SMs (gemm_2cta.cu); the row statistics of the output, when asked
     // for, come from the follow-up kernel as on every plan without an emitting epilogue

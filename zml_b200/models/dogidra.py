@@ -265,7 +265,7 @@ class _Run:
 
 
 class DogidraModel(DecoderModel):
-    KERNEL_SOURCES = ("runtime", "gemm_bf16", "gemm_2cta", "gemm_f32", "elementwise", "stream_f32", "attention", "attention_tc", "attention_prefill", "gqa_attention",
+    KERNEL_SOURCES = ("runtime", "gemm_bf16", "gemm_2cta", "gemm_stream", "gemm_f32", "elementwise", "stream_f32", "attention", "attention_tc", "attention_prefill", "gqa_attention",
                       "gated_scan", "moe", "moe_f32")
     FP32_ON_GPU = True
     # as for the other decoders with an fp32 stream: the prefill's kernels are long, overlapping their launches gains nothing

@@ -171,7 +171,7 @@ class _Layer:
 
 
 class DopuraxModel(DecoderModel):
-    KERNEL_SOURCES = ("runtime", "gemm_bf16", "gemm_2cta", "gemm_f32", "elementwise", "stream_f32", "latent_attention",
+    KERNEL_SOURCES = ("runtime", "gemm_bf16", "gemm_2cta", "gemm_stream", "gemm_f32", "elementwise", "stream_f32", "latent_attention",
                       "latent_prefill_tc", "latent_decode", "wkv", "moe")
     FP32_ON_GPU = True
     # With overlapping launches a prefill of several chunks queued back to back has stopped making progress (some kernel of
