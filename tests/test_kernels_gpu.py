@@ -342,6 +342,26 @@ def test_rope_kvwrite(layout, rot, qk_norm):
     assert torch.equal(vc, vc2)
 
 
+@pytest.mark.parametrize("hd,rot,hq,hkv,qk_norm", [(64, 64, 5, 1, True), (128, 128, 32, 8, False), (256, 64, 4, 1, True), (128, 48, 3, 3, True), (64, 16, 70, 2, False)])
+def test_rope_rows(hd, rot, hq, hkv, qk_norm):
+    """The 16-byte form: heads that do not fill a warp, more pieces than threads, partial rotation, strided input, padding rows."""
+    torch.manual_seed(hd + rot)
+    t, page, pages = 9, 64, 3
+    qkv = _randn(t, (hq + 2 * hkv) * hd + 16)[:, :(hq + 2 * hkv) * hd]
+    pos = torch.randint(0, 5000, (t,), device=DEV, dtype=torch.int32)
+    slots = torch.randperm(pages * page, device=DEV)[:t].to(torch.int32)
+    slots[4] = -1
+    inv_freq = (1.0 / (10000.0 ** (torch.arange(rot // 2, device=DEV).float() / (rot // 2)))).contiguous()
+    qn, kn = (_randn(hd), _randn(hd)) if qk_norm else (None, None)
+    kc = torch.zeros(pages, page, hkv, hd, device=DEV, dtype=torch.bfloat16)
+    vc, kc2, vc2 = kc.clone(), kc.clone(), kc.clone()
+    q = ops.rope_kvwrite(qkv, pos, slots, inv_freq, kc, vc, hq, hkv, hd, 0, rot, 1.1, qn, kn, 1e-6, qk_norm)
+    q2 = ref.rope_kvwrite(qkv, pos, slots, inv_freq, kc2, vc2, hq, hkv, hd, 0, rot, 1.1, qn, kn, 1e-6, qk_norm)
+    expect_close(q.float(), q2.float(), atol=3e-2, rtol=2e-2, min_close=0.995)
+    expect_close(kc.float(), kc2.float(), atol=3e-2, rtol=2e-2, min_close=0.995)
+    assert torch.equal(vc, vc2)
+
+
 @pytest.mark.parametrize("rows,vocab", [(1, 128256), (40, 32773), (200, 4099), (3, 1000), (2, 40)])
 def test_topk_and_argmax_over_clusters(rows, vocab):
     """Rows cut over clusters of 8, 4 and 1: random, rising, falling, all equal and lowest logits against a stable sort (equal logits: the

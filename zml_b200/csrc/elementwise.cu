@@ -246,6 +246,102 @@ __global__ void __launch_bounds__(128) zb_rope_kvwrite_kernel(const RopeParams p
   }
 }
 
+// The halves layout for heads of 64, 128 or 256 whose rows start on 16 bytes.  A CTA takes one token: its angles go to shared memory once,
+// then every thread has two 16-byte pieces of one head - the two that rotate into each other, or two behind the rotated part, or two of
+// a value head - so all loads of a token are in flight at once (the kernel above walks a warp's heads one after the other, each load
+// behind the store before it).  A head's hd / 16 threads are neighbours in a warp and add up its sum of squares.
+// 8192 tokens of 32 + 8 + 8 heads: 64 columns a head 23 us (85), 128 51 (78); 16 + 4 + 4 heads of 256, normalised, 64 columns turned 57
+// (107); 32 tokens 2.2 (3.1).
+ZB_DEVICE void rope_unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = zb_unpack_bf16x2(w[i]);
+    f[2 * i] = v.x;
+    f[2 * i + 1] = v.y;
+  }
+}
+ZB_DEVICE uint4 rope_pack8(const float (&f)[8]) {
+  return make_uint4(zb_pack_bf16x2(f[0], f[1]), zb_pack_bf16x2(f[2], f[3]), zb_pack_bf16x2(f[4], f[5]), zb_pack_bf16x2(f[6], f[7]));
+}
+
+template <int HD>
+__global__ void __launch_bounds__(512) zb_rope_rows_kernel(const RopeParams p) {
+  constexpr int kLanes = HD / 16;
+  __shared__ __align__(16) float sn[HD / 2], cs[HD / 2];
+  zb_pdl_launch();
+  zb_pdl_wait();
+  const int tok = blockIdx.x, half = p.rot_dim >> 1;
+  const float pos = static_cast<float>(p.positions[tok]);
+  const long long slot = p.slot_mapping[tok];
+  // negative = padding row (no KV write); the checking build reports a slot past the cache instead of dropping it
+  if (slot >= p.num_slots) (void)ZB_BC_OK(slot, p.num_slots, kKernelRopeKvWrite, 1);
+  const bool slot_ok = slot >= 0 && slot < p.num_slots;
+  const int units = (p.hq + 2 * p.hkv) * kLanes;
+  const int rounded = (units + 31) & ~31;            // a warp goes through the loop as a whole
+  for (int u0 = threadIdx.x; u0 < rounded; u0 += blockDim.x) {
+    const bool in = u0 < units;
+    const int u = in ? u0 : units - 1, h = u / kLanes, j = u - h * kLanes;
+    const bool is_q = h < p.hq, is_k = !is_q && h < p.hq + p.hkv;
+    const bool turns = (is_q || is_k) && j < half / 8;
+    const int v0 = turns ? j : half / 4 + 2 * (j - half / 8), v1 = turns ? j + half / 8 : v0 + 1;      // 16-byte pieces of the head
+    const int a0 = is_q || is_k ? v0 : 2 * j, a1 = is_q || is_k ? v1 : 2 * j + 1;
+    const uint4* src = reinterpret_cast<const uint4*>(p.qkv + static_cast<size_t>(tok) * p.qkv_stride + static_cast<size_t>(h) * HD);
+    uint4 x0 = src[a0], x1 = src[a1];
+    if (u0 == static_cast<int>(threadIdx.x)) {       // first turn: the angles, while the loads are on their way
+      for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        float s_, c_;
+        sincosf(pos * p.inv_freq[i], &s_, &c_);
+        sn[i] = s_ * p.attn_factor;
+        cs[i] = c_ * p.attn_factor;
+      }
+      __syncthreads();
+    }
+    if (is_q || is_k) {
+      float f0[8], f1[8];
+      rope_unpack8(x0, f0);
+      rope_unpack8(x1, f1);
+      const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
+      // q and k heads lie in front of the value heads: the lanes of one head agree, and a warp whose last lanes have values still adds
+      // up groups of kLanes
+      if (nw != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss += f0[i] * f0[i] + f1[i] * f1[i];
+        const uint32_t group = ((1ull << kLanes) - 1ull) << ((threadIdx.x & 31) / kLanes * kLanes);
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
+        const float inv = rsqrtf(ss / static_cast<float>(HD) + p.norm_eps), one = p.norm_unit_offset ? 1.f : 0.f;
+        float g0[8], g1[8];
+        rope_unpack8(reinterpret_cast<const uint4*>(nw)[a0], g0);
+        rope_unpack8(reinterpret_cast<const uint4*>(nw)[a1], g1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          // normalised in f32, rounded to the activation dtype before rotating (as the reference does)
+          f0[i] = __bfloat162float(__float2bfloat16(f0[i] * inv * (g0[i] + one)));
+          f1[i] = __bfloat162float(__float2bfloat16(f1[i] * inv * (g1[i] + one)));
+        }
+      }
+      if (turns) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float c_ = cs[8 * j + i], s_ = sn[8 * j + i], x = f0[i], y = f1[i];
+          f0[i] = x * c_ - y * s_;
+          f1[i] = y * c_ + x * s_;
+        }
+      }
+      x0 = rope_pack8(f0);
+      x1 = rope_pack8(f1);
+    }
+    if (!in || (!is_q && !slot_ok)) continue;
+    const int kvh = h - p.hq - (is_k ? 0 : p.hkv);
+    __nv_bfloat16* dst = is_q ? p.q_out + (static_cast<size_t>(tok) * p.hq + h) * HD
+                              : (is_k ? p.k_cache : p.v_cache) + (static_cast<size_t>(slot) * p.hkv + kvh) * HD;
+    reinterpret_cast<uint4*>(dst)[a0] = x0;
+    reinterpret_cast<uint4*>(dst)[a1] = x1;
+  }
+}
+
 // ---------------------------------------------------------------- SwiGLU
 // out[t, f] = silu(gu[t, f]) * gu[t, F + f]
 __global__ void __launch_bounds__(256) zb_swiglu_kernel(const __nv_bfloat16* __restrict__ gu,
@@ -691,6 +787,15 @@ int zb_rope_kvwrite(const void* qkv, void* q_out, void* k_cache, void* v_cache,
   p.norm_unit_offset = norm_unit_offset;
   p.num_slots = num_slots;
   if (rot_dim / 2 > 128) return -46;
+  const auto at16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (layout == 0 && rot_dim % 16 == 0 && (hd == 64 || hd == 128 || hd == 256) && qkv_stride % 8 == 0 && at16(qkv) && at16(q_out) && at16(k_cache) &&
+      at16(v_cache) && at16(q_norm_w) && at16(k_norm_w)) {
+    const int units = (hq + 2 * hkv) * (hd / 16), threads = units >= 512 ? 512 : (units + 31) / 32 * 32;
+    const auto kernel = hd == 64 ? zb_rope_rows_kernel<64> : (hd == 128 ? zb_rope_rows_kernel<128> : zb_rope_rows_kernel<256>);
+    zb_launch(kernel, dim3(tokens), dim3(threads), 0, reinterpret_cast<cudaStream_t>(stream), p);
+    zb_count_launch(1);
+    return static_cast<int>(cudaGetLastError());
+  }
   // enough warps to fill the SMs a few times; beyond that, more heads per warp (shared sin / cos)
   const int heads = hq + 2 * hkv;
   int heads_per_warp = static_cast<int>(static_cast<long long>(tokens) * heads / 2368);
