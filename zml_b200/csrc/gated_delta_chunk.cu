@@ -512,7 +512,7 @@ size_t zb_gated_delta_rec_bytes(int tokens, int num_seqs, int hv) { return (stat
 
 // zb_gated_delta_scan over chunks, for batches with prompts.  dk in {64, 128}; dv a multiple of 32, <= 256.  mix, z and out start on 16
 // bytes and their row strides are multiples of 8 elements.  `rec` (zb_gated_delta_rec_bytes, 16-byte aligned) and `y` (bf16
-// [tokens, hv * dv]) are scratch.
+// [tokens, hv * dv]) are scratch; y may be out.
 int zb_gated_delta_chunked(const void* mix, long long ld_mix, const void* z, long long ld_z, const void* a, const void* b, long long ld_ab,
                            const float* a_log, const float* dt_bias, const void* norm_w, float eps, float* state, void* out, long long ld_out,
                            const int32_t* q_start, const int32_t* seq_lens, const int32_t* slots, int num_seqs, int tokens, int hk, int hv, int dk,

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_kernel(const ConvParams 
 
 // The same for rows that start on 16 bytes: a thread has eight channels and walks kConvTokens tokens of one sequence, so a prompt is cut
 // along its tokens as well (8192 channels, 8192 tokens of 7 sequences: the walk of a whole sequence above took 1214 us, bound by
-// the latency of one load per token; TODO).  The inputs in front of a block are read again.  The block at a sequence's start owns
+// the latency of one load per token; 151 us).  The inputs in front of a block are read again.  The block at a sequence's start owns
 // its cache: it reads it before it writes the sequence's last inputs to it.
 constexpr int kConvTokens = 32;
 
@@ -323,6 +323,117 @@ __global__ void __launch_bounds__(256) zb_gated_delta_scan_kernel(const GdnParam
   }
 }
 
+// The same walk for few tokens per sequence - a decode step - where it is bound by reading and writing the states: a thread has four
+// columns and DK * DV / 1024 keys of the state, so that a CTA asks for its 64 KB in 16-byte pieces all at once, and q, k and the gates
+// are prepared while they come.  The key groups' partial products meet in shared memory.
+// 32 sequences of 32 heads of 128 x 128 (134 MB): 20 us (one column a thread: 34).
+template <int DK, int DV>
+__global__ void __launch_bounds__(256) zb_gated_delta_step_kernel(const GdnParams p) {
+  constexpr int kCols = DV / 4, kGroups = 256 / kCols, kKeys = DK / kGroups;
+  __shared__ __align__(16) float qk[2][DK];
+  __shared__ __align__(16) float red[2][kGroups][DV];
+  __shared__ float gates[2], ssq[8];
+  zb_pdl_launch();
+  zb_pdl_wait();
+  const int h = blockIdx.x, s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = p.q_start[s], t1 = p.q_start[s + 1];
+  if (t1 <= t0) return;
+  if (!ZB_BC_OK(p.slots[s], ZB_BC_STATE_SLOTS, kKernelGdnScan, 2)) return;      // uniform over the block
+  const bool fresh = p.seq_lens[s] - (t1 - t0) <= 0;
+  const int grp = threadIdx.x / kCols, col = (threadIdx.x - grp * kCols) * 4;
+  float* st = p.state + ((static_cast<size_t>(p.slots[s]) * p.hv + h) * DK + grp * kKeys) * DV + col;
+  float4 S[kKeys];
+#pragma unroll
+  for (int i = 0; i < kKeys; ++i) S[i] = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(st + static_cast<size_t>(i) * DV);
+  const int kh = h / (p.hv / p.hk), key_dim = p.hk * DK;
+  for (int t = t0; t < t1; ++t) {
+    const __nv_bfloat16* row = p.mix + t * p.ld_mix;
+    if (warp < 2) {                                  // q and k, normalised
+      const __nv_bfloat16* src = row + (warp == 0 ? 0 : key_dim) + kh * DK;
+      float x[DK / 32], ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < DK / 32; ++i) {
+        x[i] = __bfloat162float(src[lane + 32 * i]);
+        ss += x[i] * x[i];
+      }
+      const float inv = rsqrtf(zb_warp_sum(ss) + 1e-6f) * (warp == 0 ? rsqrtf(static_cast<float>(DK)) : 1.f);
+#pragma unroll
+      for (int i = 0; i < DK / 32; ++i) qk[warp][lane + 32 * i] = x[i] * inv;
+    } else if (warp == 2 && lane < 2) {
+      if (lane == 0) {
+        const float av = __bfloat162float(p.a[t * p.ld_ab + h]) + p.dt_bias[h];
+        gates[0] = expf(-expf(p.a_log[h]) * (av > 20.f ? av : log1pf(expf(av))));
+      } else {
+        gates[1] = 1.f / (1.f + expf(-__bfloat162float(p.b[t * p.ld_ab + h])));
+      }
+    }
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __bfloat162float(row[2 * key_dim + h * DV + col + i]);
+    __syncthreads();
+    const float alpha = gates[0], beta = gates[1];
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < kKeys; ++i) {
+      const float k = qk[1][grp * kKeys + i];
+      d[0] = fmaf(S[i].x, k, d[0]);
+      d[1] = fmaf(S[i].y, k, d[1]);
+      d[2] = fmaf(S[i].z, k, d[2]);
+      d[3] = fmaf(S[i].w, k, d[3]);
+    }
+    *reinterpret_cast<float4*>(&red[0][grp][col]) = make_float4(d[0], d[1], d[2], d[3]);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = 0.f;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+      const float4 r = *reinterpret_cast<const float4*>(&red[0][g][col]);
+      d[0] += r.x;
+      d[1] += r.y;
+      d[2] += r.z;
+      d[3] += r.w;
+    }
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = (v[i] - alpha * d[i]) * beta;
+#pragma unroll
+    for (int i = 0; i < kKeys; ++i) {
+      const float k = qk[1][grp * kKeys + i], q = qk[0][grp * kKeys + i];
+      S[i].x = alpha * S[i].x + k * d[0];
+      S[i].y = alpha * S[i].y + k * d[1];
+      S[i].z = alpha * S[i].z + k * d[2];
+      S[i].w = alpha * S[i].w + k * d[3];
+      y[0] = fmaf(S[i].x, q, y[0]);
+      y[1] = fmaf(S[i].y, q, y[1]);
+      y[2] = fmaf(S[i].z, q, y[2]);
+      y[3] = fmaf(S[i].w, q, y[3]);
+    }
+    *reinterpret_cast<float4*>(&red[1][grp][col]) = make_float4(y[0], y[1], y[2], y[3]);
+    __syncthreads();
+    // gated RMSNorm over the head's outputs, a thread per column
+    float o = 0.f;
+    if (threadIdx.x < DV) {
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) o += red[1][g][threadIdx.x];
+      o = __bfloat162float(__float2bfloat16(o));
+    }
+    const float part = zb_warp_sum(o * o);
+    if (lane == 0) ssq[warp] = part;
+    __syncthreads();
+    if (threadIdx.x < DV) {
+      float ss = 0.f;
+#pragma unroll
+      for (int w = 0; w < DV / 32; ++w) ss += ssq[w];
+      const float inv = rsqrtf(ss / static_cast<float>(DV) + p.eps);
+      const float zg = __bfloat162float(p.z[t * p.ld_z + h * DV + threadIdx.x]);
+      p.out[t * p.ld_out + h * DV + threadIdx.x] =
+          __float2bfloat16(o * inv * __bfloat162float(p.norm_w[threadIdx.x]) * (zg / (1.f + __expf(-zg))));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kKeys; ++i) *reinterpret_cast<float4*>(st + static_cast<size_t>(i) * DV) = S[i];
+}
+
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) zb_sigmoid_gate_mul_kernel(__nv_bfloat16* __restrict__ x, long long ldx,
                                                                   const __nv_bfloat16* __restrict__ gate, long long ldg,
@@ -349,6 +460,11 @@ __global__ void __launch_bounds__(256) zb_sigmoid_gate_mul_kernel(__nv_bfloat16*
 
 template <int DK>
 int launch_gdn(const GdnParams& p, int num_seqs, cudaStream_t s) {
+  if ((p.dv == 64 || p.dv == 128) && (reinterpret_cast<uintptr_t>(p.state) & 15) == 0) {
+    zb_launch(p.dv == 64 ? zb_gated_delta_step_kernel<DK, 64> : zb_gated_delta_step_kernel<DK, 128>, dim3(p.hv, num_seqs), dim3(256), 0, s, p);
+    zb_count_launch(1);
+    return static_cast<int>(cudaGetLastError());
+  }
   const int threads = (p.dv + 31) / 32 * 32;
   const size_t smem = (2 * kGdnChunk * DK + 2 * kGdnChunk * p.dv + 2 * kGdnChunk) * sizeof(float);
   static bool configured[16] = {};

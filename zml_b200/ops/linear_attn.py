@@ -90,10 +90,11 @@ def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, si
 # ---------------------------------------------------------------------------- gated delta rule
 def _delta_in_chunks(tokens: int, seqs: int) -> bool:
     """Whether a batch takes the chunked kernels (csrc/gated_delta_chunk.cu) instead of the walk token by token.  32 heads of 128, us
-    chunked / walked: 1 sequence of 8 / 16 / 64 tokens 29 / 18, 30 / 30, 30 / 101; 32 sequences of 2 / 4 / 8 / 100 tokens 49 / 39,
-    47 / 53, 50 / 86, 198 / 905; 4096 tokens 751 / 8135.  The walk takes 1.3 us a token, three launches 29 us; with many sequences both
-    are bound by the states they read and write."""
-    return tokens >= 16 * seqs or (seqs >= 16 and tokens >= 4 * seqs)
+    chunked / walked: 1 sequence of 8 / 16 / 64 tokens 27 / 17, 26 / 30, 27 / 107; 32 sequences of 2 / 4 / 8 / 100 tokens 49 / 28,
+    47 / 44, 48 / 78, 196 / 889; 4096 tokens 720 / 8179.  The walk takes 1.3 - 2 us a token, three launches 26 us; with many sequences
+    both are bound by the states they read and write."""
+    return tokens >= 16 * seqs or (seqs >= 16 and tokens >= 6 * seqs)
+
 
 
 def _rows16(x) -> bool:
@@ -150,7 +151,7 @@ def gated_delta_scan(mix, z, a, b, a_log, dt_bias, norm_w, eps, state, q_start, 
     if _delta_in_chunks(t, n) and _rows16(mix) and _rows16(z) and _rows16(out) and dk in (64, 128) and dv % 32 == 0 and dv <= 256:
         l = _lib.lib()
         rec = torch.empty(l.zb_gated_delta_rec_bytes(t, n, hv), dtype=torch.uint8, device=mix.device)
-        y = torch.empty((t, hv * dv), dtype=torch.bfloat16, device=mix.device)
+        y = out if out.stride(0) == hv * dv else torch.empty((t, hv * dv), dtype=torch.bfloat16, device=mix.device)
         rc = l.zb_gated_delta_chunked(
             _ptr(mix), mix.stride(0), _ptr(z), z.stride(0), _ptr(a), _ptr(b), a.stride(0), _ptr(a_log), _ptr(dt_bias),
             _ptr(norm_w), float(eps), _ptr(state), _ptr(out), out.stride(0), _ptr(q_start), _ptr(seq_lens),
