@@ -353,13 +353,14 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         zb_tmem_st16(t_s + 16 * c, pw);
       }
       l += zb_sum2(zb_add2(sum[0], sum[1]));
+      // Parity does not tell a phase of o_ready from the one two before it, so that no wait may begin two phases early or end two late: the
+      // last tile but one is waited for while the last one is still held back.
+      if (j > 0 && j == n_tiles - 1) ok = zb_mbar_wait(&o_ready[w], static_cast<uint32_t>(j - 1) & 1u, abort_flag);
       zb_tmem_st_wait();
       zb_tc_fence_before();
       __syncwarp();
       if (lane == 0) zb_mbar_arrive(&p_full[w]);
     }
-    // the last two tiles' O += P V, in this order: parity alone does not tell a phase from the one two before it
-    if (ok && n_tiles > 1) ok = zb_mbar_wait(&o_ready[w], static_cast<uint32_t>(n_tiles - 2) & 1u, abort_flag);
     if (ok && n_tiles > 0) ok = zb_mbar_wait(&o_ready[w], static_cast<uint32_t>(n_tiles - 1) & 1u, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) {
       *abort_where = 14u + w;
