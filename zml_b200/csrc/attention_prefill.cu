@@ -110,8 +110,8 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* v_full = k_full + kStages;               // kStages
   uint64_t* kv_empty = v_full + kStages;             // kStages, both heads' MMAs
   uint64_t* s_full = kv_empty + kStages;             // [2 heads][2 buffers]
-  uint64_t* p_full = s_full + 4;                     // 2, four warps
-  uint64_t* o_ready = p_full + 2;                    // 2
+  uint64_t* p_full = s_full + 4;                     // [2 heads][2 buffers], four warps
+  uint64_t* o_ready = p_full + 4;                    // 2
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_ready + 2);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
@@ -156,11 +156,10 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     for (int i = 0; i < 4; ++i) {
       zb_mbar_init(&s_full[i], 1);
+      zb_mbar_init(&p_full[i], 4);
     }
-    for (int w = 0; w < 2; ++w) {
-      zb_mbar_init(&p_full[w], 4);
-      zb_mbar_init(&o_ready[w], 1);
-    }
+    zb_mbar_init(&o_ready[0], 1);
+    zb_mbar_init(&o_ready[1], 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -241,7 +240,8 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           where = 4u;
           break;
         }
-        if (!zb_mbar_wait(&p_full[w], static_cast<uint32_t>(j) & 1u, abort_flag)) {
+        // (a barrier per buffer: the softmax may publish the next tile's P before this one's V has come)
+        if (!zb_mbar_wait(&p_full[2 * w + (j & 1)], static_cast<uint32_t>(j >> 1) & 1u, abort_flag)) {
           where = 5u;
           break;
         }
@@ -359,7 +359,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       zb_tmem_st_wait();
       zb_tc_fence_before();
       __syncwarp();
-      if (lane == 0) zb_mbar_arrive(&p_full[w]);
+      if (lane == 0) zb_mbar_arrive(&p_full[2 * w + b]);
     }
     if (ok && n_tiles > 0) ok = zb_mbar_wait(&o_ready[w], static_cast<uint32_t>(n_tiles - 1) & 1u, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) {
