@@ -294,7 +294,7 @@ def test_paged_prefill_tensor_core_kernel(hq, hkv, lens):
         expect_close(got.float(), old.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
 
 
-@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("lens", [[(1, 0), (63, 0), (64, 1), (65, 63)], [(127, 0), (128, 64), (129, 191)], [(3, 4000), (260, 0)]])
 def test_paged_prefill_page_edges(hd, lens):
     """The tcgen05 prefill kernels at the edges of pages and query blocks, with scores that grow along the keys, so that a row's

@@ -1,11 +1,11 @@
-// Paged prefill attention without extensions on the 5th-generation tensor cores (tcgen05 / TMEM / TMA): head_dim 64 and 128,
-// 64-token KV pages, grouped-query attention with an even group size.
+// Paged prefill attention without extensions on the 5th-generation tensor cores (tcgen05 / TMEM / TMA): head_dim 64, 128 and
+// 256, 64-token KV pages, grouped-query attention (with an even group size up to 128).
 //
-// One CTA works on 128 query rows of TWO query heads that share a KV head; every page that it brings in feeds both heads' softmax
-// pipelines:
+// One CTA works on 128 query rows of TWO query heads that share a KV head - of one head where head_dim is 256 - and every page that it
+// brings in feeds both heads' softmax pipelines:
 //   warps 0-3 / 4-7 : softmax and epilogue of head A / B, one thread per query row
-//   warp  8         : TMA producer (Q once, then K and V pages through a ring)
-//   warps 9, 10     : one thread each issues the MMAs of head A / B, so that neither head waits for the other's events
+//   next warp       : TMA producer (Q once, then K and V pages through a ring)
+//   last warps      : one thread each issues the MMAs of head A / B, so that neither head waits for the other's events
 // Per page and head: S = Q K^T (fp32 in tensor memory), P = 2^(S - m) as bf16 over S, O += P V (A = P from tensor memory, B = V in
 // its natural [key][head_dim] layout, MN-major).
 //
@@ -19,7 +19,9 @@
 //   * a few exponentials run as polynomials on the FMA pipes (Shape::kPoly).
 // 8192 queries on 16384 keys, 32 heads on 8: head_dim 128 1.35 ms (1220 TFLOP/s; the kernel before it: 2.33), head_dim 64 1.19 ms (694;
 // the mma.sync kernel: 5.17).  4 x 2048: 0.18 (0.29) and 0.15 (0.48) ms.
-// Tensor memory columns: S_A 0 and 64 | S_B 128 and 192 (P in the first half of each) | O_A 256 | O_B 384.
+// Tensor memory columns: S_A 0 and 64 | S_B 128 and 192 (P in the first half of each) | O_A 256 | O_B 384, or one O from 256 on.
+// head_dim 256: 1024 clocks of multiply-adds a page cover the softmax of one head; its O leaves no room for another's.  16 heads on 4:
+// 8192 tokens 0.80 ms (689 TFLOP/s; the mma.sync kernel: 4.64), seven prompts of 128 to 2048 tokens 0.19 (0.88) ms.
 // Every wait is bounded; a wait that runs out records a status and the CTA leaves through its normal exit.
 #include <cuda.h>
 
@@ -74,16 +76,17 @@ struct PrefillParams {
 
 template <int HD>
 struct Shape {
-  static constexpr int kStages = HD == 64 ? 8 : 5;
+  static constexpr int kStages = HD == 64 ? 8 : (HD == 128 ? 5 : 2);
+  static constexpr int kHeads = HD == 256 ? 1 : 2;                 // of a CTA
+  static constexpr int kThreads = 32 * (5 * kHeads + 1);
   static constexpr int kSubs = HD / 64;                            // 64-column sub-tiles
   static constexpr int kQBytes = kRows * HD * 2, kKvBytes = kKeys * HD * 2;
   // Of 16 pairs of exponentials, those that the FMA pipes take.  8192 queries on 16384 keys, 32 heads: head_dim 64 0 / 4 / 6 / 8 pairs
   // 1246 / 1189 / 1270 / 1357 us, head_dim 128 0 / 1 / 4 1380 / 1352 / 1395 us.  More of them fill the ALU pipe (cuts, exponents).
   static constexpr int kPoly = HD == 64 ? 4 : 1;
-  static constexpr int kSmem = 2 * kQBytes + 2 * kStages * kKvBytes + 1024 + 256;
+  static constexpr int kSmem = kHeads * kQBytes + 2 * kStages * kKvBytes + 1024 + 256;
 };
-constexpr uint32_t kColS = 0, kColO = 256;           // S: [head][buffer][64], O: [head][128]
-constexpr int kThreads = 352;
+constexpr uint32_t kColS = 0, kColO = 256;           // S: [head][buffer][64], O: [head][128] or [256]
 
 // max of three, one instruction
 ZB_DEVICE float max3(float a, float b, float c) {
@@ -93,16 +96,16 @@ ZB_DEVICE float max3(float a, float b, float c) {
 }
 
 template <int HD>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<HD>::kThreads, 1)
 zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   using S = Shape<HD>;
-  constexpr int kStages = S::kStages;
+  constexpr int kStages = S::kStages, kHeads = S::kHeads;
   zb_pdl_wait();                                     // q, the KV cache and the batch description come from preceding work
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* q_s = smem;                               // [2 heads][kQBytes]
-  uint8_t* k_s = q_s + 2 * S::kQBytes;               // [kStages][kKvBytes]
+  uint8_t* q_s = smem;                               // [kHeads][kQBytes]
+  uint8_t* k_s = q_s + kHeads * S::kQBytes;               // [kStages][kKvBytes]
   uint8_t* v_s = k_s + kStages * S::kKvBytes;        // [kStages][kKvBytes]
   uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + kStages * S::kKvBytes);
   uint64_t* q_full = bars;                           // 1
@@ -118,7 +121,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.num_q_heads / p.num_kv_heads;
-  const int head0 = blockIdx.x * 2;
+  const int head0 = blockIdx.x * kHeads;
   const int kvh = head0 / group;
 
   // The (sequence, 128-row query block) of this CTA.  Head pairs are the grid's fast index, and blocks are handed out from the end of
@@ -152,7 +155,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     for (int s = 0; s < kStages; ++s) {
       zb_mbar_init(&k_full[s], 1);
       zb_mbar_init(&v_full[s], 1);
-      zb_mbar_init(&kv_empty[s], 2);
+      zb_mbar_init(&kv_empty[s], kHeads);
     }
     for (int i = 0; i < 4; ++i) {
       zb_mbar_init(&s_full[i], 1);
@@ -167,7 +170,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     zb_tma_prefetch_desc(&tmap_k);
     zb_tma_prefetch_desc(&tmap_v);
   }
-  if (warp == 9) {
+  if (warp == 4 * kHeads + 1) {
     zb_tmem_alloc(tmem_holder, kTmemCols);
     zb_tmem_relinquish();
   }
@@ -177,12 +180,12 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const uint32_t tmem_base = *tmem_holder;
   zb_pdl_launch();                                   // only now: a successor that also takes tensor memory must not come first
 
-  if (warp == 8) {
+  if (warp == 4 * kHeads) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
-      zb_mbar_expect_tx(q_full, 2 * S::kQBytes);
-      for (int w = 0; w < 2; ++w)
+      zb_mbar_expect_tx(q_full, kHeads * S::kQBytes);
+      for (int w = 0; w < kHeads; ++w)
         for (int c = 0; c < S::kSubs; ++c)
           zb_tma_load_2d(q_s + w * S::kQBytes + c * (kRows * 128), &tmap_q, q_full, (head0 + w) * HD + c * 64, tok_base);
       uint32_t stage = 0, phase = 0;
@@ -203,10 +206,10 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         }
       }
     }
-  } else if (warp > 8) {
+  } else if (warp > 4 * kHeads) {
     // ------------------------------------------------------------------ MMA issuer of head w
     if (lane == 0) {
-      const int w = warp - 9;
+      const int w = warp - 4 * kHeads - 1;
       constexpr uint32_t kIdescS = zb_make_idesc_bf16(kRows, kKeys);
       constexpr uint32_t kIdescO = zb_make_idesc_bf16(kRows, HD) | (1u << 16);         // B (= V) is MN-major
       const uint32_t t_s = tmem_base + kColS + w * 128, t_o = tmem_base + kColO + w * 128;
@@ -396,7 +399,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == 4 * kHeads + 1) {
     zb_tc_fence_after();
     zb_tmem_dealloc(tmem_base, kTmemCols);
   }
@@ -406,7 +409,7 @@ template <int HD>
 int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int q_blocks, cudaStream_t s) {
   static bool configured[16] = {};
   if (const int rc = zb_config_smem_once(zb_prefill_kernel<HD>, Shape<HD>::kSmem, configured)) return rc;
-  const cudaError_t le = zb_launch(zb_prefill_kernel<HD>, dim3(p.num_q_heads / 2, q_blocks), dim3(kThreads), Shape<HD>::kSmem, s, tq, tk, tv, p);
+  const cudaError_t le = zb_launch(zb_prefill_kernel<HD>, dim3(p.num_q_heads / Shape<HD>::kHeads, q_blocks), dim3(Shape<HD>::kThreads), Shape<HD>::kSmem, s, tq, tk, tv, p);
   zb_count_launch(1);
   return static_cast<int>(le != cudaSuccess ? le : cudaGetLastError());
 }
@@ -436,5 +439,6 @@ int zb_prefill_plain(const void* q, const void* k_cache, const void* v_cache, vo
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (head_dim == 256) return launch_prefill<256>(tq, tk, tv, p, q_blocks, s);
   return head_dim == 64 ? launch_prefill<64>(tq, tk, tv, p, q_blocks, s) : launch_prefill<128>(tq, tk, tv, p, q_blocks, s);
 }

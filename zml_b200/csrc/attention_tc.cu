@@ -613,11 +613,11 @@ constexpr int kSmemBytes = 2 * kQBytes + 2 * kStages * kKvBytes + 1024 + 256;
 
 extern "C" {
 
-// 1 when a tensor-core prefill kernel takes this shape (head_dim 128, without ZbAttnExt also 64; 64-token pages, an even number of
-// query heads per KV head), else 0: the caller then uses the mma.sync kernel.
+// 1 when a tensor-core prefill kernel takes this shape (head_dim 128, without ZbAttnExt also 64 and 256; 64-token pages, up to 128 an even
+// number of query heads per KV head), else 0: the caller then uses the mma.sync kernel.
 int zb_paged_prefill_tc_supported(int num_q_heads, int num_kv_heads, int head_dim, int page_size) {
-  if ((head_dim != kHD && head_dim != 64) || page_size != kKeys || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
-  return ((num_q_heads / num_kv_heads) % 2) == 0 ? 1 : 0;
+  if ((head_dim != kHD && head_dim != 64 && head_dim != 256) || page_size != kKeys || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
+  return head_dim == 256 || ((num_q_heads / num_kv_heads) % 2) == 0 ? 1 : 0;
 }
 
 // 1 when the kernel takes a call with ZbAttnExt: no cap, or one whose exponential fp32 holds; differential heads without a cap.

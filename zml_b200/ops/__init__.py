@@ -389,7 +389,7 @@ def _ext(ext):
     return None if ext is None else C.addressof(ext)
 
 
-# ZB_ATTN_TC=0: prefill attention always on the mma.sync kernel (the tensor-core kernels take head_dim 64 and 128,
+# ZB_ATTN_TC=0: prefill attention always on the mma.sync kernel (the tensor-core kernels take head_dim 64, 128 and 256,
 # 64-token pages and an even number of query heads per KV head)
 import os as _os
 _ATTN_TC = _os.environ.get("ZB_ATTN_TC", "1") != "0"
@@ -398,7 +398,7 @@ _ATTN_TC = _os.environ.get("ZB_ATTN_TC", "1") != "0"
 def _tc_takes(q, k_cache, ext) -> bool:
     l = _lib.lib()
     ok = bool(l.zb_paged_prefill_tc_supported(q.shape[1], k_cache.shape[2], q.shape[2], k_cache.shape[1])) and q.stride(0) % 8 == 0
-    if q.shape[2] == 64 and ext is None:            # tensor maps start on 16 bytes; the mma.sync kernel takes other pointers
+    if q.shape[2] != 128 and ext is None:           # tensor maps start on 16 bytes; the mma.sync kernel takes other pointers
         return ok and (q.data_ptr() | k_cache.data_ptr()) % 16 == 0
     return ok and (ext is None or (q.shape[2] == 128 and bool(l.zb_paged_prefill_tc_ext_supported(ext.cap, ext.pair))))
 
