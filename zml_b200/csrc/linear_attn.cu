@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_kernel(const ConvParams 
 
 // The same for rows that start on 16 bytes: a thread has eight channels and walks kConvTokens tokens of one sequence, so a prompt is cut
 // along its tokens as well (8192 channels, 8192 tokens of 7 sequences: the walk of a whole sequence above took 1214 us, bound by
-// the latency of one load per token; 151 us).  The inputs in front of a block are read again.  The block at a sequence's start owns
+// the latency of one load per token; 141 us).  The inputs in front of a block are read again.  The block at a sequence's start owns
 // its cache: it reads it before it writes the sequence's last inputs to it.
 constexpr int kConvTokens = 32;
 
@@ -161,32 +161,36 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const Conv
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) *reinterpret_cast<uint4*>(st + static_cast<size_t>(j) * p.channels) = last[j];
   }
-#pragma unroll 4
-  for (int t = a; t < b; ++t) {
-    float x[8], acc[8];
-    input(t, x);
+  for (int t4 = a; t4 < b; t4 += 4) {                // four tokens' inputs on their way at once
+    float x4[4][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float v = w[K - 1][i] * x[i];
+    for (int q = 0; q < 4; ++q) input(min(t4 + q, b - 1), x4[q]);
 #pragma unroll
-      for (int j = 0; j < K - 1; ++j) v += w[j][i] * win[j][i];
-      v = conv_round(v);
-      if (p.silu) v = v / (1.f + __expf(-v));
-      acc[i] = v;
+    for (int q = 0; q < 4; ++q) {
+      const int t = t4 + q;
+      if (t >= b) break;
+      float acc[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float v = w[K - 1][i] * x4[q][i];
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) v += w[j][i] * (q + j < K - 1 ? win[q + j][i] : x4[q + j - (K - 1)][i]);
+        v = conv_round(v);
+        if (p.silu) v = v / (1.f + __expf(-v));
+        acc[i] = v;
+      }
+      if (p.post != nullptr) {
+        float g[8];
+        conv_unpack8(*reinterpret_cast<const uint4*>(p.post + t * p.ldpost + c), g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = conv_round(acc[i]) * g[i];
+      }
+      *reinterpret_cast<uint4*>(p.out + t * p.ldo + c) = conv_pack8(acc);
     }
 #pragma unroll
-    for (int j = 0; j + 1 < K - 1; ++j)
+    for (int j = 0; j < K - 1; ++j)                  // K - 1 <= 4: the window in front of the next four
 #pragma unroll
-      for (int i = 0; i < 8; ++i) win[j][i] = win[j + 1][i];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) win[K - 2][i] = x[i];
-    if (p.post != nullptr) {
-      float g[8];
-      conv_unpack8(*reinterpret_cast<const uint4*>(p.post + t * p.ldpost + c), g);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = conv_round(acc[i]) * g[i];
-    }
-    *reinterpret_cast<uint4*>(p.out + t * p.ldo + c) = conv_pack8(acc);
+      for (int i = 0; i < 8; ++i) win[j][i] = x4[4 - (K - 1) + j][i];
   }
 }
 
@@ -502,7 +506,7 @@ int zb_causal_conv1d(const void* x, long long ldx, const void* pre, long long ld
   p.silu = silu;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const auto at16 = [](const void* q, long long ld) { return q == nullptr || ((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld & 7) == 0); };
-  if (channels % 8 == 0 && at16(x, ldx) && at16(pre, ldpre) && at16(post, ldpost) && at16(out, ldo) && at16(state, 0) &&
+  if (out != x && out != pre && channels % 8 == 0 && at16(x, ldx) && at16(pre, ldpre) && at16(post, ldpost) && at16(out, ldo) && at16(state, 0) &&
       tokens / kConvTokens + num_seqs <= 65535) {
     const dim3 blocks((channels / 8 + 127) / 128, tokens / kConvTokens + num_seqs);
     switch (kernel_size) {
