@@ -2,16 +2,20 @@
 //
 // The work is to read the weights once.  The tcgen05 kernel (gemm_bf16.cu) streams them well once it runs, but each launch pays for
 // barriers, tensor memory, descriptors, a ring of tiles through shared memory and a cluster reduction, about 8 us that a matrix of 8 MB
-// (1.3 us at the copy bandwidth) does not have.  Here a CTA takes 16 weight rows at a time with 8 warps along K; weights go from
-// global memory straight into the registers of mma.sync (m16n8k16, weights as A, the tokens as the 8 columns of B):
+// (1.3 us at the copy bandwidth) does not have.  Here a CTA takes 16 weight rows at a time with 8 warps along K, on mma.sync (m16n8k16,
+// weights as A, the tokens as the 8 columns of B):
 //   * K is summed in an order of our own.  A lane's 16-byte piece of a weight row is four pairs of consecutive columns, which are its
-//     A operands of two MMAs; the same 16 bytes of a token's row are its B operands.  No shuffles, no shared memory.
-//   * A warp owns 128 columns of every 1024 (256 bytes a row) and keeps two such groups of 16 rows on their way: 16 KB a warp.
-//   * With static weights both groups are requested before the kernel in front has finished (programmatic dependent launch); only the
-//     tokens wait for it.
+//     A operands of two MMAs; the same 16 bytes of a token's row are its B operands.  No shuffles, no barriers.
+//   * A warp owns 128 columns of every 1024 (256 bytes a row) and keeps kDepth such groups of 16 rows on their way, by cp.async into a
+//     ring of which every thread reads what it asked for itself.  (Straight into registers they need room in the L1 cache while they
+//     come, and a launch that starts under a kernel with the largest shared memory finds almost none: a decode step of the 8B model with
+//     4 sequences took 3.6 ms, with the ring 1.73; on the tcgen05 kernel 2.26.)
+//   * With static weights the ring is requested before the kernel in front has finished (programmatic dependent launch); only the tokens
+//     wait for it.  A grid that one CTA per SM can do asks for more than half of an SM's shared memory: CTAs that start early, while
+//     the kernel in front still holds most SMs, would otherwise crowd on the others.
 // The warps' sums meet in shared memory, once per 16 rows.
-// One token, us (tcgen05 kernel; weights at the copy bandwidth): 2048 x 2048 2.9 (7.3; 1.3), 3072 x 2048 3.2 (8.0; 1.9), 16384 x 2048 with
-// SwiGLU 10.7 (17.1; 10.1), 2048 x 8192 9.1 (13.0; 5.0), 28672 x 4096 35.6 (43.0; 35.3); eight tokens 0.3 - 3 more.
+// One token, us (tcgen05 kernel; weights at the copy bandwidth): 2048 x 2048 3.1 (7.3; 1.3), 3072 x 2048 3.4 (8.0; 1.9), 16384 x 2048 with
+// SwiGLU 10.7 (17.1; 10.1), 2048 x 8192 8.2 (13.0; 5.0), 28672 x 4096 36.9 (43.0; 35.3); eight tokens 0.4 - 4 more.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -22,6 +26,9 @@
 namespace {
 constexpr int kWarps = 8, kRowsTile = 16, kTokens = 8, kGroup = 4;       // 32-column blocks of a warp's group
 constexpr int kSpan = kWarps * kGroup * 32;                              // columns that the CTA's groups cover
+constexpr int kDepth = 3;
+constexpr int kRing = kDepth * 2 * kGroup * 32 * kWarps * 16;            // 96 KB
+constexpr int kOnePerSm = 120 * 1024;                                    // shared memory of which two CTAs do not fit an SM
 
 struct StreamParams {
   const __nv_bfloat16* w;
@@ -37,10 +44,8 @@ struct StreamParams {
   float in_inv_d, in_eps;
 };
 
-ZB_DEVICE uint4 ld_stream(const __nv_bfloat16* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
+ZB_DEVICE void copy16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16u : 0u) : "memory");
 }
 ZB_DEVICE void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -49,6 +54,7 @@ ZB_DEVICE void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
 }
 
 __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const StreamParams p) {
+  extern __shared__ __align__(16) uint4 ring[];      // [kDepth][2 kGroup][threads]
   __shared__ float part[2][kWarps][kTokens][kRowsTile + 1];
   __shared__ float scale[kTokens];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
@@ -59,20 +65,25 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   const int col0 = warp * (kGroup * 32) + tq * 8;
   // position of the next group to request
-  int l_tile = blockIdx.x, l_group = 0;
-  auto request = [&](uint4 (&lo)[kGroup], uint4 (&hi)[kGroup]) {
-    const int r0 = l_tile * kRowsTile + g, c = l_group * kSpan + col0;
-    const __nv_bfloat16* at = p.w + static_cast<long long>(r0) * p.ldw + c;
+  int l_tile = blockIdx.x, l_group = 0, l_left = steps;
+  auto request = [&](int slot) {
+    if (l_left > 0) {
+      --l_left;
+      const int r0 = l_tile * kRowsTile + g, c = l_group * kSpan + col0;
+      const __nv_bfloat16* at = p.w + static_cast<long long>(r0) * p.ldw + c;
+      const uint32_t to = zb_smem_u32(ring + slot * (2 * kGroup * 32 * kWarps) + threadIdx.x);
 #pragma unroll
-    for (int u = 0; u < kGroup; ++u) {
-      const bool in = c + 32 * u < p.k;
-      lo[u] = in && r0 < p.n ? ld_stream(at + 32 * u) : zero;
-      hi[u] = in && r0 + 8 < p.n ? ld_stream(at + 8 * p.ldw + 32 * u) : zero;
+      for (int u = 0; u < kGroup; ++u) {
+        const bool in = c + 32 * u < p.k, lo = in && r0 < p.n, hi = in && r0 + 8 < p.n;
+        copy16(to + (2 * u) * (32 * kWarps * 16), lo ? at + 32 * u : p.w, lo);
+        copy16(to + (2 * u + 1) * (32 * kWarps * 16), hi ? at + 8 * p.ldw + 32 * u : p.w, hi);
+      }
+      if (++l_group == groups) {
+        l_group = 0;
+        l_tile += gridDim.x;
+      }
     }
-    if (++l_group == groups) {
-      l_group = 0;
-      l_tile += gridDim.x;
-    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int x_group = 0;
   auto request_x = [&](uint4 (&x)[kGroup]) {
@@ -82,16 +93,11 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
       x[u] = g < p.m && c + 32 * u < p.k ? *reinterpret_cast<const uint4*>(p.a + static_cast<long long>(g) * p.lda + c + 32 * u) : zero;
     if (++x_group == groups) x_group = 0;
   };
-  uint4 lo[2][kGroup], hi[2][kGroup], x[2][kGroup];
-  if (p.static_w) {
-    request(lo[0], hi[0]);
-    if (steps > 1) request(lo[1], hi[1]);
-    zb_pdl_wait();
-  } else {
-    zb_pdl_wait();
-    request(lo[0], hi[0]);
-    if (steps > 1) request(lo[1], hi[1]);
-  }
+  uint4 x[2][kGroup];
+  if (!p.static_w) zb_pdl_wait();
+#pragma unroll
+  for (int i = 0; i < kDepth; ++i) request(i);
+  if (p.static_w) zb_pdl_wait();
   request_x(x[0]);
   if (steps > 1) request_x(x[1]);
   if (p.in_sumsq != nullptr) {                       // warp t: RMSNorm factor of token t
@@ -106,16 +112,19 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
   int tile = blockIdx.x, group = 0, buf = 0;
   const int tok = threadIdx.x >> 3, pair = threadIdx.x & 7;              // of the first 64 threads: outputs (tok, 2 pair .. 2 pair + 1)
   float ss_out = 0.f;
-  auto step = [&](uint4 (&l)[kGroup], uint4 (&h)[kGroup], uint4 (&xx)[kGroup], int s) {
+  int slot = 0;
+  auto step = [&](uint4 (&xx)[kGroup], int s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+    const uint4* mine_in = ring + slot * (2 * kGroup * 32 * kWarps) + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
-      mma16816(acc[0], l[u].x, h[u].x, l[u].y, h[u].y, xx[u].x, xx[u].y);
-      mma16816(acc[1], l[u].z, h[u].z, l[u].w, h[u].w, xx[u].z, xx[u].w);
+      const uint4 l = mine_in[(2 * u) * (32 * kWarps)], h = mine_in[(2 * u + 1) * (32 * kWarps)];
+      mma16816(acc[0], l.x, h.x, l.y, h.y, xx[u].x, xx[u].y);
+      mma16816(acc[1], l.z, h.z, l.w, h.w, xx[u].z, xx[u].w);
     }
-    if (s + 2 < steps) {
-      request(l, h);
-      request_x(xx);
-    }
+    request(slot);                                   // behind the reads of what it overwrites
+    if (++slot == kDepth) slot = 0;
+    if (s + 2 < steps) request_x(xx);
     if (++group < groups) return;
     group = 0;
 #pragma unroll
@@ -161,8 +170,8 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
     tile += gridDim.x;
   };
   for (int s = 0; s < steps; s += 2) {
-    step(lo[0], hi[0], x[0], s);
-    if (s + 1 < steps) step(lo[1], hi[1], x[1], s + 1);
+    step(x[0], s);
+    if (s + 1 < steps) step(x[1], s + 1);
   }
   if (p.out_sumsq != nullptr && threadIdx.x < 64) {
 #pragma unroll
@@ -208,7 +217,9 @@ int zb_gemm_stream_launch(const void* a, const void* w, void* out, const void* r
   // row statistics: one part per CTA, of which a consumer takes 160 at most
   const int grid = std::min(p.tiles, p.out_sumsq != nullptr ? num_sms : 2 * num_sms);
   if (out_parts != nullptr && p.out_sumsq != nullptr) *out_parts = grid;
-  const cudaError_t e = zb_launch(zb_gemm_stream_kernel, dim3(grid), dim3(32 * kWarps), 0, stream, p);
+  static bool configured[16] = {};
+  if (const int rc = zb_config_smem_once(zb_gemm_stream_kernel, kOnePerSm, configured)) return rc;
+  const cudaError_t e = zb_launch(zb_gemm_stream_kernel, dim3(grid), dim3(32 * kWarps), grid > num_sms ? kRing : kOnePerSm, stream, p);
   zb_count_launch(1);
   return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
