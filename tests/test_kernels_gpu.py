@@ -138,6 +138,26 @@ def test_gemm_few_tokens(m, n, k):
         expect_close(act.float(), torch.nn.functional.silu(sc[:, :n // 2]) * sc[:, n // 2:], atol=2e-2, rtol=2e-2, min_close=ALL)
 
 
+@pytest.mark.parametrize("m,n,k", [(100, 5128, 2048), (129, 264, 72), (200, 136, 2048), (257, 264, 64), (512, 2048, 576), (300, 3080, 712), (770, 5128, 1024)])
+def test_gemm_pair_tiles(m, n, k):
+    """The two-SM kernel's three tile widths with ragged last tiles, from the fewest tokens it takes on (one shape of too few columns for
+    it), its statistics and SwiGLU; also behind a kernel that writes its input, with the weights requested early."""
+    torch.manual_seed(n)
+    a, w, res = _randn(m, k), _randn(n, k, scale=1.0 / math.sqrt(k)), _randn(m, n)
+    base = a.float() @ w.float().t()
+    out, stats = ops.gemm(a, w, residual=res, emit_stats=True, static_w=True)
+    expect_close(out.float(), base + res.float(), atol=3e-2, rtol=2e-2, min_close=ALL)
+    expect_close(stats.total(), out.float().pow(2).sum(-1), atol=1e-2, rtol=1e-4, min_close=ALL)
+    scale = torch.rsqrt(a.float().pow(2).mean(-1, keepdim=True) + 1e-5)
+    b = torch.empty_like(a)
+    for _ in range(3):
+        b.copy_(a)
+        sc = base * scale
+        act = ops.gemm(b, ops.interleave_gate_up(w), row_stats=ops.row_sumsq(b), swiglu=True, static_w=True)
+        expect_close(act.float(), torch.nn.functional.silu(sc[:, :n // 2]) * sc[:, n // 2:], atol=3e-2, rtol=2e-2, min_close=ALL)
+        b.zero_()
+
+
 @pytest.mark.parametrize("rows,d", [(1, 2048), (33, 4096), (64, 8192), (5, 1024 + 8), (3, 16384)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm(rows, d, with_res):

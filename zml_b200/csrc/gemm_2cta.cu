@@ -19,6 +19,7 @@
 // epilogue of a tile overlaps the main loop of the next one).  Every wait is bounded.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -29,16 +30,21 @@ int zb_make_tmap_bf16_2d(CUtensorMap* out, const void* base, int rows, int k, in
 namespace {
 
 constexpr int kBM = 128;          // rows of A per CTA (256 per pair)
-constexpr int kBNH = 128;         // rows of W per CTA (the pair's tile is 256 columns wide)
-constexpr int kBN = 2 * kBNH;
 constexpr int kBK = 64;
-constexpr int kStages = 6;
-constexpr int kStageBytes = (kBM + kBNH) * kBK * 2;          // 32 KB
 constexpr int kTileABytes = kBM * kBK * 2;
 constexpr int kThreads = 192;
 constexpr int kEpiThreads = 128;
 constexpr uint32_t kKernelId = 14;
-constexpr uint32_t kTmemCols = 512;                           // two accumulator stages of 256 fp32 columns
+// A pair's tile is 256 rows by BN = 256, 128 or 64 columns; each CTA loads BN / 2 rows of W.  Two accumulator stages of BN fp32 columns.
+template <int BN>
+struct Tile {
+  static constexpr int kBNH = BN / 2;
+  static constexpr int kStageBytes = (kBM + kBNH) * kBK * 2;
+  static constexpr int kStages = BN == 256 ? 6 : (BN == 128 ? 8 : 10);
+  static constexpr uint32_t kTmemCols = 2 * BN;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+};
+constexpr int kMaxParts = 160;                                // row statistics: parts that a consumer's buffer holds
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;               // clears the CTA-rank bit of a shared::cluster address
 
 struct Gemm2Params {
@@ -48,9 +54,10 @@ struct Gemm2Params {
   const __nv_bfloat16* residual;
   const __nv_bfloat16* bias;
   int out_f32;
-  int num_m, num_n;             // tiles of 256 x 256
+  int static_w;                 // W may be read before the kernel in front is done
+  int num_m, num_n;             // tiles of 256 x BN
   int group_m;                  // rasterisation: tiles of `group_m` consecutive row blocks share their W tiles in L2
-  ZbGemmEpi epi;                // row scale (in_sumsq, in_parts, in_ld, in_inv_d, in_eps) and swiglu are honoured
+  ZbGemmEpi epi;                // all but pf_*; out_sumsq has a part per tile column
   ZbStatus* status;
 };
 
@@ -93,8 +100,12 @@ ZB_DEVICE void mbar_arrive_remote(uint32_t cluster_addr) {
 ZB_DEVICE void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 ZB_DEVICE float silu2(float g) { return g / (1.f + __expf(-g)); }
 
+template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const Gemm2Params prm) {
+  using T = Tile<BN>;
+  constexpr int kStages = T::kStages, kStageBytes = T::kStageBytes, kBNH = T::kBNH, kBN = BN;
+  constexpr uint32_t kTmemCols = T::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
@@ -151,13 +162,25 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   zb_cluster_wait();
   const uint32_t tmem_base = *tmem_holder;
   zb_pdl_launch();
-  zb_pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
+      // static weights: those of the first ring of stages are on their way before the kernel in front is done
+      int early = 0;
+      if (prm.static_w && cluster_id < num_tiles) {
+        int mt, nt;
+        decode(cluster_id, mt, nt);
+        early = min(kStages, kb_total);
+        for (int kb = 0; kb < early; ++kb) {
+          if (cta_rank == 0) zb_mbar_expect_tx(&full_bar[kb], 2 * kStageBytes);
+          tma_load_2d_pair(smem + kb * kStageBytes + kTileABytes, &tmap_w, zb_smem_u32(&full_bar[kb]) & kPeerBitMask, kb * kBK,
+                           nt * kBN + static_cast<int>(cta_rank) * kBNH);
+        }
+      }
+      zb_pdl_wait();
       for (int t = cluster_id; ok && t < num_tiles; t += n_clusters) {
         int mt, nt;
         decode(t, mt, nt);
@@ -171,9 +194,13 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           uint8_t* sa = smem + stage * kStageBytes;
           const uint32_t lbar = zb_smem_u32(&full_bar[stage]) & kPeerBitMask;
-          if (cta_rank == 0) zb_mbar_expect_tx(&full_bar[stage], 2 * kStageBytes);       // both CTAs' bytes
+          if (early > 0) {
+            --early;
+          } else {
+            if (cta_rank == 0) zb_mbar_expect_tx(&full_bar[stage], 2 * kStageBytes);     // both CTAs' bytes
+            tma_load_2d_pair(sa + kTileABytes, &tmap_w, lbar, kb * kBK, row_w);
+          }
           tma_load_2d_pair(sa, &tmap_a, lbar, kb * kBK, row_a);
-          tma_load_2d_pair(sa + kTileABytes, &tmap_w, lbar, kb * kBK, row_w);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -219,6 +246,7 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else {
     // ------------------------------------------------------------ epilogue: this CTA's 128 rows of the tile
+    zb_pdl_wait();                                   // residual, row statistics, and whoever still reads what is written here
     const int epi_tid = threadIdx.x - 64;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
@@ -241,6 +269,7 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (*abort_flag != 0u) break;
       zb_tc_fence_after();
       const uint32_t taddr = tmem_base + acc * kBN + (static_cast<uint32_t>(quad * 32) << 16);
+      float ss_out = 0.f;
 #pragma unroll 1
       for (int c0 = 0; c0 < kBN; c0 += 32) {
         uint32_t r[32];
@@ -312,17 +341,30 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         } else {
           __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(prm.out) + o;
           if (whole) {
+            uint32_t w[16];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              reinterpret_cast<uint4*>(op)[i] = make_uint4(zb_pack_bf16x2(v[8 * i], v[8 * i + 1]), zb_pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                                                           zb_pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), zb_pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+            for (int j = 0; j < 16; ++j) w[j] = zb_pack_bf16x2(v[2 * j], v[2 * j + 1]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(op)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+            if (prm.epi.out_sumsq != nullptr) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float2 f = zb_unpack_bf16x2(w[j]);
+                ss_out = fmaf(f.x, f.x, fmaf(f.y, f.y, ss_out));
+              }
+            }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (q + j < prm.n) op[j] = __float2bfloat16(v[j]);
+              if (q + j < prm.n) {
+                const __nv_bfloat16 b = __float2bfloat16(v[j]);
+                op[j] = b;
+                ss_out = fmaf(__bfloat162float(b), __bfloat162float(b), ss_out);
+              }
           }
         }
       }
+      if (prm.epi.out_sumsq != nullptr && p < prm.m) prm.epi.out_sumsq[static_cast<size_t>(nt) * prm.epi.out_ld + p] = ss_out;
       // this CTA has read accumulator stage `acc`: one arrival on the leader's barrier
       zb_tc_fence_before();
       epi_sync();
@@ -351,34 +393,55 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
 }
 
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+// Columns of the tiles.  A k-block takes 0.35 us with 256 columns and 0.31 with 64 (256 rows of A have to come either way), so narrow tiles
+// pay only where more SMs share the problem in the same single wave: 512 x 2048 x 2048 20.9 -> 15.3 us with the statistics, 512 x 3072 x
+// 2048 17.1 -> 15.3; but 1024 x 6144 x 4096 in three waves of 128 columns 62 us, in two of 256 46.
+int tile_columns(int m, int n, int num_sms) {
+  const long long mt = (m + 2 * kBM - 1) / (2 * kBM);
+  int bn = 256;
+  while (bn > 64 && mt * ((n + bn / 2 - 1) / (bn / 2)) <= num_sms / 2) bn >>= 1;
+  return bn;
+}
+
+template <int BN>
+int launch_tiles(const CUtensorMap& ta, const void* w, int ldw, Gemm2Params prm, int num_sms, cudaStream_t stream) {
+  static bool configured[16] = {};
+  if (const int rc = zb_config_smem_once(zb_gemm_2cta_kernel<BN>, Tile<BN>::kSmemBytes, configured)) return rc;
+  CUtensorMap tw;
+  if (const int rc = zb_make_tmap_bf16_2d(&tw, w, prm.n, prm.k, ldw, BN / 2)) return rc;
+  prm.num_m = (prm.m + 2 * kBM - 1) / (2 * kBM);
+  prm.num_n = (prm.n + BN - 1) / BN;
+  const int clusters = std::min(num_sms / 2, prm.num_m * prm.num_n);
+  const cudaError_t le = zb_launch_cluster(zb_gemm_2cta_kernel<BN>, dim3(2 * clusters), dim3(kThreads), Tile<BN>::kSmemBytes, stream, 2, ta, tw, prm);
+  zb_count_launch(1);
+  return static_cast<int>(le != cudaSuccess ? le : cudaGetLastError());
+}
 
 }  // namespace
 
-// 1 when the two-SM kernel takes the problem: tokens as rows (more than 256 of them) and at least one full tile of
-// columns.  ZB_GEMM_2CTA=0 in the environment turns the kernel off.
-int zb_gemm_2cta_wants(int m, int n, int k) {
+// 1 when the two-SM kernel takes the problem: tokens as rows and at least one full tile of columns.  Above 128 tokens always (200 tokens, us,
+// here / one-SM kernel with weights as rows: 5120 x 2048 15 / 55, 28672 x 4096 60 / 139, 4096 x 14336 68 / 105).  From 65 on where the
+// estimates say so - a wave of tiles 0.32 us a k-block, the one-SM kernel 0.7 us for each k-block of 128 x 128 that an SM has to do and 7
+// more to begin with: 128 tokens, us: 5120 x 2048 15.1 / 17.1, 28672 x 4096 58 / 91, 2048 x 4096 22.6 / 16.0, 4096 x 14336 68 / 35.
+// ZB_GEMM_2CTA=0 in the environment turns the kernel off.
+int zb_gemm_2cta_wants(int m, int n, int k, int num_sms) {
   static int enabled = -1;
   if (enabled < 0) {
     const char* e = getenv("ZB_GEMM_2CTA");
     enabled = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
-  return enabled && m >= 512 && n >= 256 && k >= 64;
+  if (!enabled || m <= 64 || n < 256 || k < 64) return 0;
+  if (m > 128) return 1;
+  const int bn = tile_columns(m, n, num_sms), kb = (k + kBK - 1) / kBK;
+  const int waves = ((n + bn - 1) / bn + num_sms / 2 - 1) / (num_sms / 2);
+  return 0.32 * waves * kb < 7. + 0.7 * ((n + 127) / 128) * kb / num_sms;
 }
 
 // out[M,N] = a[M,K] * w[N,K]^T (* row scale) (+ bias) (+ residual) or its SwiGLU: same contract as the one-SM
-// kernel's launch for the options it supports (epi->out_sumsq and epi->pf_* are ignored here; the caller
-// handles them).  Returns 0 on success.
+// kernel's launch (epi->pf_* is ignored).  `out_parts`: parts written to epi->out_sumsq.  Returns 0 on success.
 int zb_gemm_2cta_launch(const void* a, const void* w, void* out, const void* residual, const void* bias, int m, int n, int k, int lda,
-                        int ldw, int ldo, int out_f32, const ZbGemmEpi* epi, ZbStatus* status, int num_sms, cudaStream_t stream) {
-  static bool configured[16] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return -21;
-  if (!configured[dev]) {
-    cudaError_t e = zb_config_smem(zb_gemm_2cta_kernel, kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured[dev] = true;
-  }
+                        int ldw, int ldo, int out_f32, int static_w, const ZbGemmEpi* epi, int* out_parts, ZbStatus* status, int num_sms,
+                        cudaStream_t stream) {
   Gemm2Params prm = {};
   prm.m = m;
   prm.n = n;
@@ -388,20 +451,18 @@ int zb_gemm_2cta_launch(const void* a, const void* w, void* out, const void* res
   prm.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   prm.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   prm.out_f32 = out_f32 & 1;
-  prm.num_m = (m + 2 * kBM - 1) / (2 * kBM);
-  prm.num_n = (n + kBN - 1) / kBN;
+  prm.static_w = static_w;
   prm.group_m = 8;
   if (epi != nullptr) prm.epi = *epi;
   prm.status = status;
-  CUtensorMap ta, tw;
-  int rc = zb_make_tmap_bf16_2d(&ta, a, m, k, lda, kBM);
-  if (rc != 0) return rc;
-  rc = zb_make_tmap_bf16_2d(&tw, w, n, k, ldw, kBNH);
-  if (rc != 0) return rc;
-  const int tiles = prm.num_m * prm.num_n;
-  int clusters = num_sms / 2;
-  if (clusters > tiles) clusters = tiles;
-  const cudaError_t le = zb_launch_cluster(zb_gemm_2cta_kernel, dim3(2 * clusters), dim3(kThreads), kSmemBytes, stream, 2, ta, tw, prm);
-  zb_count_launch(1);
-  return static_cast<int>(le != cudaSuccess ? le : cudaGetLastError());
+  int bn = tile_columns(m, n, num_sms);
+  if (prm.epi.out_sumsq != nullptr) {
+    while (bn < 256 && (n + bn - 1) / bn > kMaxParts) bn *= 2;
+    if (out_parts != nullptr) *out_parts = (n + bn - 1) / bn;
+  }
+  CUtensorMap ta;
+  if (const int rc = zb_make_tmap_bf16_2d(&ta, a, m, k, lda, kBM)) return rc;
+  if (bn == 64) return launch_tiles<64>(ta, w, ldw, prm, num_sms, stream);
+  if (bn == 128) return launch_tiles<128>(ta, w, ldw, prm, num_sms, stream);
+  return launch_tiles<256>(ta, w, ldw, prm, num_sms, stream);
 }

@@ -1675,7 +1675,9 @@ void zb_set_l2_prefetch_mb(int mb) { g_l2_prefetch_mb = mb < 0 ? 0 : (mb > 96 ? 
 int zb_gemm_plan(int m, int n, int k, int num_sms, int split_hint, int* swap, int* bn, int* grid,
                  int* units_per_cta, int* rr_tiles) {
   const int kb_total = (k + kBlockK - 1) / kBlockK;
-  const int sw = m <= 256 ? 1 : 0;
+  // Weights as the tile's rows up to 256 tokens; of so few weight rows that the tokens fill more tiles (a router), up to 128: 200 tokens of
+  // 128 x 2048 as one 128 x 256 tile cut along K took 49 us.
+  const int sw = m <= (n < 256 && split_hint <= 0 ? 128 : 256) ? 1 : 0;
   int b;
   if (sw) {
     b = 16;
@@ -1725,9 +1727,10 @@ size_t zb_gemm_workspace_bytes(int m, int n, int k, int num_sms) {
 int zb_gemm_stream_wants(const void* a, const void* w, int m, int n, int k);
 int zb_gemm_stream_launch(const void* a, const void* w, void* out, const void* residual, const void* bias, int m, int n, int k, int lda, int ldw,
                           int ldo, int out_f32, int static_w, const ZbGemmEpi* epi, int* out_parts, int num_sms, cudaStream_t stream);
-int zb_gemm_2cta_wants(int m, int n, int k);
+int zb_gemm_2cta_wants(int m, int n, int k, int num_sms);
 int zb_gemm_2cta_launch(const void* a, const void* w, void* out, const void* residual, const void* bias, int m, int n, int k, int lda,
-                        int ldw, int ldo, int out_f32, const ZbGemmEpi* epi, ZbStatus* status, int num_sms, cudaStream_t stream);
+                        int ldw, int ldo, int out_f32, int static_w, const ZbGemmEpi* epi, int* out_parts, ZbStatus* status, int num_sms,
+                        cudaStream_t stream);
 
 namespace {
 
@@ -1771,11 +1774,15 @@ int gemm_impl(const void* a, const void* w, void* out, const void* residual, con
   if (rc != 0) return rc;
   if ((band == nullptr || band->mode == 0) && split_hint <= 0 && zb_gemm_stream_wants(a, w, m, n, k))
     return zb_gemm_stream_launch(a, w, out, residual, bias, m, n, k, lda, ldw, ldo, out_f32, static_w, epi, out_parts, num_sms, stream);
-  if ((band == nullptr || band->mode == 0) && split_hint <= 0 && zb_gemm_2cta_wants(m, n, k)) {
-    // prefill-sized: 256 x 256 tiles on pairs of SMs (gemm_2cta.cu); the row statistics of the output, when asked
-    // for, come from the follow-up kernel as on every plan without an emitting epilogue
-    rc = zb_gemm_2cta_launch(a, w, out, residual, bias, m, n, k, lda, ldw, ldo, out_f32, epi, status, num_sms, stream);
-    if (rc == 0 && epi != nullptr && epi->out_sumsq != nullptr) {
+  if ((band == nullptr || band->mode == 0) && split_hint <= 0 && zb_gemm_2cta_wants(m, n, k, num_sms)) {
+    // prefill-sized: tiles on pairs of SMs (gemm_2cta.cu).  An output of so many columns that its row statistics would have too many parts
+    // takes them from the follow-up kernel.
+    const bool after = epi != nullptr && epi->out_sumsq != nullptr && (n + 255) / 256 > 160;
+    ZbGemmEpi own = epi != nullptr ? *epi : ZbGemmEpi{};
+    if (after) own.out_sumsq = nullptr;
+    rc = zb_gemm_2cta_launch(a, w, out, residual, bias, m, n, k, lda, ldw, ldo, out_f32, static_w, epi != nullptr ? &own : nullptr, out_parts, status,
+                             num_sms, stream);
+    if (rc == 0 && after) {
       if (out_parts) *out_parts = 1;
       rc = launch_row_sumsq(out, m, n, ldo, epi->out_sumsq, stream);
     }
