@@ -451,6 +451,19 @@ def test_moe_combine_adds_extra_and_residual():
     expect_close(cpu.float(), want.cpu(), atol=3e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("t,k,d", [(511, 8, 64), (512, 1, 2056), (515, 9, 1024), (700, 8, 4104)])
+def test_moe_gather_by_tokens(t, k, d):
+    """The expert rows gathered from the tokens' side (from 512 tokens on) are those of the gather by rows, half of the experts elsewhere."""
+    from zml_b200 import moe
+    torch.manual_seed(t)
+    x, ids = _randn(t, d), torch.stack([torch.randperm(16, device=DEV)[:k] for _ in range(t)]).int()
+    meta, sorted_pair, pair_pos = moe.moe_align(ids, 4, 8)
+    rows = int(meta[8])
+    want = x[sorted_pair[:rows].long() // k]
+    assert torch.equal(moe.gather(x, sorted_pair, meta, 8, k, t * k, pair_pos)[:rows], want)
+    assert torch.equal(moe.gather(x, sorted_pair, meta, 8, k, t * k)[:rows], want)
+
+
 @pytest.mark.parametrize("tokens", [1, 333, 1365, 3000])       # up to 8192 pairs: one launch; above: count / prefix / scatter
 def test_moe_align_is_a_permutation(tokens):
     from zml_b200 import moe

@@ -326,6 +326,30 @@ __global__ void __launch_bounds__(128) zb_moe_gather_kernel(const __nv_bfloat16*
   }
 }
 
+// The same from the tokens' side, for batches with prompts: a CTA reads its token's row once and stores it to the rows of the token's
+// pairs, all independent of each other (by position every row's load waits for the pair behind it).  8192 tokens of 2048, 8 experts
+// each: 51 us (80).
+__global__ void __launch_bounds__(128) zb_moe_spread_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pair_pos,
+                                                            __nv_bfloat16* __restrict__ xs, int k, int d) {
+  zb_pdl_launch();
+  zb_pdl_wait();
+  const size_t t = blockIdx.x;
+  const int nvec = d / 8;
+  const uint4* src = reinterpret_cast<const uint4*>(x) + t * nvec;
+  for (int i = threadIdx.x; i < nvec; i += 256) {
+    const bool two = i + 128 < nvec;
+    const uint4 v0 = src[i], v1 = two ? src[i + 128] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) {
+      const int pos = pair_pos[t * k + j];
+      if (pos < 0) continue;
+      uint4* dst = reinterpret_cast<uint4*>(xs) + static_cast<size_t>(pos) * nvec;
+      dst[i] = v0;
+      if (two) dst[i + 128] = v1;
+    }
+  }
+}
+
 // The gather with the NVFP4 activation quantiser behind it: xq[pos, :] = e2m1 codes of x[sorted_pair[pos] / k, :],
 // xsf[pos, :] = one f8e4m3 scale per 16 values (same numerics as zb_nvfp4_quantize without a per-tensor scale).
 // One thread per 16-value block.
@@ -425,17 +449,29 @@ zb_moe_combine_kernel(const __nv_bfloat16* __restrict__ o, const int32_t* __rest
   bool timed_out = false;
   for (int i = threadIdx.x; i < nvec; i += 128) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < k; ++j) {
-      const int pos = pair_pos[static_cast<size_t>(t) * k + j];
-      if (pos < 0) continue;
-      const float w = weights[static_cast<size_t>(t) * k + j];
-      const uint4 v = reinterpret_cast<const uint4*>(o + static_cast<size_t>(pos) * d)[i];
-      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    for (int j0 = 0; j0 < k; j0 += 8) {              // eight rows on their way at once (60 against 76 us for 8192 tokens of 2048), added up in order
+      int pos[8];
+      float w[8];
+      uint4 v[8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 f = zb_unpack_bf16x2(u[q]);
-        acc[2 * q] += w * f.x;
-        acc[2 * q + 1] += w * f.y;
+      for (int j = 0; j < 8; ++j) {
+        const bool in = j0 + j < k;
+        pos[j] = in ? pair_pos[static_cast<size_t>(t) * k + j0 + j] : -1;
+        w[j] = in ? weights[static_cast<size_t>(t) * k + j0 + j] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = pos[j] >= 0 ? reinterpret_cast<const uint4*>(o + static_cast<size_t>(pos[j]) * d)[i] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (pos[j] < 0) continue;
+        const uint32_t u[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = zb_unpack_bf16x2(u[q]);
+          acc[2 * q] += w[j] * f.x;
+          acc[2 * q + 1] += w[j] * f.y;
+        }
       }
     }
     if (extra != nullptr) {
@@ -903,6 +939,16 @@ int zb_moe_gather(const void* x, const int32_t* sorted_pair, const int32_t* meta
   int blocks = cap < 2368 ? cap : 2368;
   zb_launch(zb_moe_gather_kernel, dim3(blocks), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream), 
       reinterpret_cast<const __nv_bfloat16*>(x), sorted_pair, meta, reinterpret_cast<__nv_bfloat16*>(xs), e_local, k, d, cap);
+  zb_count_launch(1);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The same from pair_pos (`zb_moe_align`): one CTA per token.  xs has a row for every local pair.
+int zb_moe_spread(const void* x, const int32_t* pair_pos, void* xs, int tokens, int k, int d, void* stream) {
+  if (tokens <= 0) return 0;
+  if (d % 8 != 0) return -62;
+  zb_launch(zb_moe_spread_kernel, dim3(tokens), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __nv_bfloat16*>(x), pair_pos,
+            reinterpret_cast<__nv_bfloat16*>(xs), k, d);
   zb_count_launch(1);
   return static_cast<int>(cudaGetLastError());
 }

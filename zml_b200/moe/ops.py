@@ -14,6 +14,7 @@ _lib.register_signature("zb_moe_align", C.c_int, [C.c_void_p, C.c_void_p, C.c_vo
                                                    C.c_int, C.c_void_p], optional=False)
 _lib.register_signature("zb_moe_gather", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
                                                     C.c_int, C.c_int, C.c_void_p], optional=False)
+_lib.register_signature("zb_moe_spread", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p], optional=False)
 _lib.register_signature("zb_moe_finalize", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
                                                       C.c_int, C.c_void_p], optional=False)
 _lib.register_signature("zb_moe_grouped_gemm", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
@@ -120,8 +121,13 @@ def moe_align(ids: torch.Tensor, e0: int, e_local: int):
     return meta, sorted_pair, pair_pos
 
 
-def gather(x: torch.Tensor, sorted_pair: torch.Tensor, meta: torch.Tensor, e_local: int, k: int, cap: int):
-    """xs[pos] = x[sorted_pair[pos] // k] for the rows in use; xs has `cap` rows."""
+# tokens from which `gather` goes by tokens instead of by rows: their CTAs fill the GPU
+SPREAD_TOKENS = 512
+
+
+def gather(x: torch.Tensor, sorted_pair: torch.Tensor, meta: torch.Tensor, e_local: int, k: int, cap: int,
+           pair_pos: Optional[torch.Tensor] = None):
+    """xs[pos] = x[sorted_pair[pos] // k] for the rows in use; xs has `cap` rows.  `pair_pos`: of `moe_align`."""
     d = x.shape[1]
     if not x.is_cuda:
         n = int(meta[e_local])
@@ -129,6 +135,9 @@ def gather(x: torch.Tensor, sorted_pair: torch.Tensor, meta: torch.Tensor, e_loc
         xs[:n] = x[(sorted_pair[:n].long() // k)]
         return xs
     xs = torch.empty((cap, d), dtype=x.dtype, device=x.device)
+    if pair_pos is not None and x.shape[0] >= SPREAD_TOKENS and cap >= pair_pos.numel() and x.is_contiguous():
+        _lib.check(_lib.lib().zb_moe_spread(x.data_ptr(), pair_pos.data_ptr(), xs.data_ptr(), x.shape[0], k, d, _lib.stream_ptr()), "zb_moe_spread")
+        return xs
     _lib.check(_lib.lib().zb_moe_gather(x.data_ptr(), sorted_pair.data_ptr(), meta.data_ptr(), xs.data_ptr(), e_local,
                                         k, d, cap, _lib.stream_ptr()), "zb_moe_gather")
     return xs
@@ -555,7 +564,7 @@ def expert_rows(x: torch.Tensor, topk_ids: torch.Tensor, w_gate_up_il: torch.Ten
     if x.is_cuda and x.dtype == torch.float32:
         h = _grouped_f32(x, sorted_pair, k, w_gate_up_il, meta, t * k, t, activation_code(activation), limits)
         return _grouped_f32(h, None, 1, w_down, meta, t * k, t, 0), pair_pos
-    xs = gather(x, sorted_pair, meta, e_local, k, t * k)
+    xs = gather(x, sorted_pair, meta, e_local, k, t * k, pair_pos)
     h = grouped_gemm(xs, w_gate_up_il, meta, swiglu=activation, avg_tokens=avg, limits=limits)
     return grouped_gemm(h, w_down, meta, swiglu=False, avg_tokens=avg), pair_pos
 
@@ -586,7 +595,7 @@ def fused_experts(x: torch.Tensor, topk_ids: torch.Tensor, topk_w: torch.Tensor,
         if extra is None and residual is None and fused is None:
             return finalize(o, pair_pos, topk_w, t, k)
         return combine(o, pair_pos, topk_w, t, k, extra, residual, fused)
-    xs = gather(x, sorted_pair, meta, e_local, k, cap)
+    xs = gather(x, sorted_pair, meta, e_local, k, cap, pair_pos)
     if w4 is not None and avg <= W4_MAX_AVG_TOKENS and w4[0].kernel_ready and w4[1].kernel_ready:
         # few tokens per expert: the step is bound by reading expert weights - read them as NVFP4
         h = grouped_gemm_w4(xs, w4[0], meta, swiglu=activation, avg_tokens=avg)
