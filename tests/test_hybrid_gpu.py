@@ -166,6 +166,20 @@ def _cpu_twin(gpu, name):
     return cpu
 
 
+@pytest.mark.parametrize("tokens", [1, 9, 130, 300])
+def test_mlp_on_interleaved_rows(tokens):
+    """The gated MLP of a dense hybrid layer against float32 from the weights that its checkpoint names hold."""
+    m = registry.build_model("tiny-qwen35-test", device=DEV, seed=5)
+    sd, lw = m.state_dict_hf(), m.layers[0]
+    torch.manual_seed(tokens)
+    x, n2 = (torch.randn(tokens, m.config.hidden_size, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    gate, up, down = (next(v for k, v in sd.items() if k.endswith(f"layers.0.mlp.{w}_proj.weight")).float() for w in ("gate", "up", "down"))
+    act = (torch.nn.functional.silu(n2.float() @ gate.t()) * (n2.float() @ up.t())).bfloat16()
+    # one rounding of the activation on either side, one of the result: 2^-8 of each, and of the sum's largest terms
+    want = x.float() + act.float() @ down.t()          # first: the residual is added in place
+    expect_close(m.mlp(lw, x, n2).float(), want, atol=1e-2, rtol=1e-2, min_close=1 - 1e-9)
+
+
 @pytest.mark.parametrize("name", ["tiny-qwen35-test", "tiny-qwen35-moe-test", "tiny-lfm2-test"])
 def test_hybrid_prefill_logits_match_cpu(name):
     from zml_b200.models.llama import AttnMeta

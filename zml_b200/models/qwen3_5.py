@@ -193,7 +193,7 @@ class Qwen35Model(LlamaModel):
         c, d = self.config, self.config.hidden_size
         g = rw((c.intermediate_size, d), b + 4, rows=self.f_rng)
         u = rw((c.intermediate_size, d), b + 5, rows=self.f_rng)
-        lw.gate_up = torch.cat([g, u], 0)
+        self._set_gate_up(lw, g, u)
         lw.down = rw((d, c.intermediate_size), b + 6, cols=self.f_rng)
 
     def init_random(self, seed: int = 0, std: float = 0.02, full: Optional[bool] = None) -> "Qwen35Model":
@@ -246,8 +246,7 @@ class Qwen35Model(LlamaModel):
         return self
 
     def _load_mlp(self, lw: LayerWeights, get, has, p: str) -> None:
-        lw.gate_up = torch.cat([get(p + "mlp.gate_proj.weight", rows=self.f_rng),
-                                get(p + "mlp.up_proj.weight", rows=self.f_rng)], 0)
+        self._set_gate_up(lw, get(p + "mlp.gate_proj.weight", rows=self.f_rng), get(p + "mlp.up_proj.weight", rows=self.f_rng))
         lw.down = get(p + "mlp.down_proj.weight", cols=self.f_rng)
 
     def load(self, store, prefix: Optional[str] = None) -> "Qwen35Model":
@@ -295,8 +294,9 @@ class Qwen35Model(LlamaModel):
         return self
 
     def _mlp_state_dict(self, lw: LayerWeights, p: str, out: dict) -> None:
-        out[p + "mlp.gate_proj.weight"] = lw.gate_up[:self.f_local]
-        out[p + "mlp.up_proj.weight"] = lw.gate_up[self.f_local:]
+        gate, up = (lw.gate_up[0::2].contiguous(), lw.gate_up[1::2].contiguous()) if self._interleaved(lw) else lw.gate_up.split(self.f_local)
+        out[p + "mlp.gate_proj.weight"] = gate
+        out[p + "mlp.up_proj.weight"] = up
         out[p + "mlp.down_proj.weight"] = lw.down
 
     def state_dict_hf(self) -> dict:
@@ -343,6 +343,30 @@ class Qwen35Model(LlamaModel):
         return n
 
     # ------------------------------------------------------------------ forward
+    def _set_gate_up(self, lw: LayerWeights, gate: torch.Tensor, up: torch.Tensor) -> None:
+        """On a GPU as rows (gate_0, up_0, gate_1, ...): SwiGLU then runs in the epilogue of the GEMM (8192 tokens of 12288: 120 us a
+        layer less than with a pass of its own).  The layer carries its layout, so that a copy of it keeps it."""
+        if self.device.type == "cuda" and self.dtype == torch.bfloat16:
+            lw.gate_up = torch.stack([gate, up], 1).flatten(0, 1)
+            lw.extra = dict(lw.extra or {}, gate_up_interleaved=True)
+        else:
+            lw.gate_up = torch.cat([gate, up], 0)
+
+    @staticmethod
+    def _interleaved(lw: LayerWeights) -> bool:
+        return bool(lw.extra) and "gate_up_interleaved" in lw.extra
+
+    def mlp(self, lw: LayerWeights, x, n2):
+        if not self._interleaved(lw):
+            return super().mlp(lw, x, n2)
+        from ..ops import baseline as _baseline
+        if _baseline.enabled():
+            gu = ops.gemm(n2, lw.gate_up)
+            act = ops.swiglu(torch.cat([gu[:, 0::2], gu[:, 1::2]], 1))
+        else:
+            act = ops.gemm(n2, lw.gate_up, static_w=True, swiglu=True)
+        return self.row_parallel(act, lw.down, x)
+
     def _seq_meta(self, meta: AttnMeta, tokens: int):
         """(q_start, seq_lens, slots) of this launch; decode steps are one token per sequence."""
         if meta.state_slots is None:
