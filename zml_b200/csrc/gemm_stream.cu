@@ -1,9 +1,9 @@
-// out[M,N] = a[M,K] * w[N,K]^T for at most 8 tokens: the decode step of a few sequences.
+// out[M,N] = a[M,K] * w[N,K]^T for at most 8 tokens, 16 for smaller matrices: the decode step of a few sequences.
 //
 // The work is to read the weights once.  The tcgen05 kernel (gemm_bf16.cu) streams them well once it runs, but each launch pays for
 // barriers, tensor memory, descriptors, a ring of tiles through shared memory and a cluster reduction, about 8 us that a matrix of 8 MB
 // (1.3 us at the copy bandwidth) does not have.  Here a CTA takes 16 weight rows at a time with 8 warps along K, on mma.sync (m16n8k16,
-// weights as A, the tokens as the 8 columns of B):
+// weights as A, tokens as the 8 columns of B, one or two such tiles):
 //   * K is summed in an order of our own.  A lane's 16-byte piece of a weight row is four pairs of consecutive columns, which are its
 //     A operands of two MMAs; the same 16 bytes of a token's row are its B operands.  No shuffles, no barriers.
 //   * A warp owns 128 columns of every 1024 (256 bytes a row) and keeps kDepth such groups of 16 rows on their way, by cp.async into a
@@ -24,7 +24,9 @@
 #include "host_api.h"
 
 namespace {
-constexpr int kWarps = 8, kRowsTile = 16, kTokens = 8, kGroup = 4;       // 32-column blocks of a warp's group
+constexpr int kWarps = 8, kRowsTile = 16, kGroup = 4;                    // 32-column blocks of a warp's group
+constexpr int kMaxTokens = 16;
+constexpr long long kMaxLarge = 20ll << 20;                             // elements of a matrix for more than 8 tokens
 constexpr int kSpan = kWarps * kGroup * 32;                              // columns that the CTA's groups cover
 constexpr int kDepth = 3;
 constexpr int kRing = kDepth * 2 * kGroup * 32 * kWarps * 16;            // 96 KB
@@ -53,10 +55,12 @@ ZB_DEVICE void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// TT: tiles of 8 tokens
+template <int TT>
 __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint4 ring[];      // [kDepth][2 kGroup][threads]
-  __shared__ float part[2][kWarps][kTokens][kRowsTile + 1];
-  __shared__ float scale[kTokens];
+  __shared__ float part[2][kWarps][8 * TT][kRowsTile + 1];
+  __shared__ float scale[8 * TT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
   zb_pdl_launch();
   const int groups = (p.k + kSpan - 1) / kSpan;
@@ -86,41 +90,49 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   int x_group = 0;
-  auto request_x = [&](uint4 (&x)[kGroup]) {
+  auto request_x = [&](uint4 (&x)[TT][kGroup]) {
     const int c = x_group * kSpan + col0;
 #pragma unroll
-    for (int u = 0; u < kGroup; ++u)
-      x[u] = g < p.m && c + 32 * u < p.k ? *reinterpret_cast<const uint4*>(p.a + static_cast<long long>(g) * p.lda + c + 32 * u) : zero;
+    for (int t = 0; t < TT; ++t)
+#pragma unroll
+      for (int u = 0; u < kGroup; ++u)
+        x[t][u] = g + 8 * t < p.m && c + 32 * u < p.k ? *reinterpret_cast<const uint4*>(p.a + static_cast<long long>(g + 8 * t) * p.lda + c + 32 * u) : zero;
     if (++x_group == groups) x_group = 0;
   };
-  uint4 x[2][kGroup];
+  uint4 x[2][TT][kGroup];
   if (!p.static_w) zb_pdl_wait();
 #pragma unroll
   for (int i = 0; i < kDepth; ++i) request(i);
   if (p.static_w) zb_pdl_wait();
   request_x(x[0]);
   if (steps > 1) request_x(x[1]);
-  if (p.in_sumsq != nullptr) {                       // warp t: RMSNorm factor of token t
-    float ss = 0.f;
-    if (warp < p.m)
-      for (int i = lane; i < p.in_parts; i += 32) ss += p.in_sumsq[static_cast<size_t>(i) * p.in_ld + warp];
-    ss = zb_warp_sum(ss);
-    if (lane == 0) scale[warp] = rsqrtf(ss * p.in_inv_d + p.in_eps);
+  if (p.in_sumsq != nullptr) {                       // warp t: RMSNorm factor of tokens t, t + 8
+#pragma unroll
+    for (int t = warp; t < 8 * TT; t += kWarps) {
+      float ss = 0.f;
+      if (t < p.m)
+        for (int i = lane; i < p.in_parts; i += 32) ss += p.in_sumsq[static_cast<size_t>(i) * p.in_ld + t];
+      ss = zb_warp_sum(ss);
+      if (lane == 0) scale[t] = rsqrtf(ss * p.in_inv_d + p.in_eps);
+    }
   }
 
-  float acc[2][4] = {};
+  float acc[TT][2][4] = {};
   int tile = blockIdx.x, group = 0, buf = 0;
-  const int tok = threadIdx.x >> 3, pair = threadIdx.x & 7;              // of the first 64 threads: outputs (tok, 2 pair .. 2 pair + 1)
+  const int tok = threadIdx.x >> 3, pair = threadIdx.x & 7;              // of the first 64 TT threads: outputs (tok, 2 pair .. 2 pair + 1)
   float ss_out = 0.f;
   int slot = 0;
-  auto step = [&](uint4 (&xx)[kGroup], int s) {
+  auto step = [&](uint4 (&xx)[TT][kGroup], int s) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
     const uint4* mine_in = ring + slot * (2 * kGroup * 32 * kWarps) + threadIdx.x;
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
       const uint4 l = mine_in[(2 * u) * (32 * kWarps)], h = mine_in[(2 * u + 1) * (32 * kWarps)];
-      mma16816(acc[0], l.x, h.x, l.y, h.y, xx[u].x, xx[u].y);
-      mma16816(acc[1], l.z, h.z, l.w, h.w, xx[u].z, xx[u].w);
+#pragma unroll
+      for (int t = 0; t < TT; ++t) {
+        mma16816(acc[t][0], l.x, h.x, l.y, h.y, xx[t][u].x, xx[t][u].y);
+        mma16816(acc[t][1], l.z, h.z, l.w, h.w, xx[t][u].z, xx[t][u].w);
+      }
     }
     request(slot);                                   // behind the reads of what it overwrites
     if (++slot == kDepth) slot = 0;
@@ -128,12 +140,14 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
     if (++group < groups) return;
     group = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      part[buf][warp][2 * tq + (i & 1)][g + 8 * (i >> 1)] = acc[0][i] + acc[1][i];
-      acc[0][i] = acc[1][i] = 0.f;
-    }
+    for (int t = 0; t < TT; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        part[buf][warp][8 * t + 2 * tq + (i & 1)][g + 8 * (i >> 1)] = acc[t][0][i] + acc[t][1][i];
+        acc[t][0][i] = acc[t][1][i] = 0.f;
+      }
     __syncthreads();                                 // the other buffer is read by nobody any more once all warps are here
-    if (threadIdx.x < 64 && tok < p.m) {
+    if (threadIdx.x < 64 * TT && tok < p.m) {
       const int row = tile * kRowsTile + 2 * pair;
       float v[2] = {0.f, 0.f};
 #pragma unroll
@@ -173,7 +187,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
     step(x[0], s);
     if (s + 1 < steps) step(x[1], s + 1);
   }
-  if (p.out_sumsq != nullptr && threadIdx.x < 64) {
+  if (p.out_sumsq != nullptr && threadIdx.x < 64 * TT) {
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) ss_out += __shfl_xor_sync(0xffffffffu, ss_out, o);
     if (pair == 0 && tok < p.m) p.out_sumsq[static_cast<size_t>(blockIdx.x) * p.out_ld + tok] = ss_out;
@@ -181,9 +195,12 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
 }
 }  // namespace
 
-// 1 when the kernel takes the problem.
+// 1 when the kernel takes the problem.  9 to 16 tokens double the tokens' reads (as many bytes as the weights) and the MMAs, which a large
+// matrix does not hide.  12 / 16 tokens, us (tcgen05 kernel): 2048 x 2048 3.9 / 4.1 (7.5), 5120 x 2048 8.4 / 9.7 (9.9), 2048 x 8192
+// 9.8 / 10.5 (13.1), 4096 x 4096 10.4 / 11.3 (12.4); 6144 x 4096 15.0 / 16.7 (16.5), 16384 x 2048 16.8 / 19.7 (17.5), 28672 x 4096
+// 49.2 / 55.5 (44.2): the line lies between the last two groups.
 int zb_gemm_stream_wants(const void* a, const void* w, int m, int n, int k) {
-  return m <= kTokens && n >= 16 && k >= 64 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+  return (m <= 8 || (m <= kMaxTokens && static_cast<long long>(n) * k <= kMaxLarge)) && n >= 16 && k >= 64 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 
 // The contract of the tcgen05 kernel's launch; epi->pf_* is ignored.  `out_parts`: parts written to epi->out_sumsq.
@@ -217,9 +234,12 @@ int zb_gemm_stream_launch(const void* a, const void* w, void* out, const void* r
   // row statistics: one part per CTA, of which a consumer takes 160 at most
   const int grid = std::min(p.tiles, p.out_sumsq != nullptr ? num_sms : 2 * num_sms);
   if (out_parts != nullptr && p.out_sumsq != nullptr) *out_parts = grid;
-  static bool configured[16] = {};
-  if (const int rc = zb_config_smem_once(zb_gemm_stream_kernel, kOnePerSm, configured)) return rc;
-  const cudaError_t e = zb_launch(zb_gemm_stream_kernel, dim3(grid), dim3(32 * kWarps), grid > num_sms ? kRing : kOnePerSm, stream, p);
+  const auto launch = [&](auto kernel, bool (&configured)[16]) {
+    if (const int rc = zb_config_smem_once(kernel, kOnePerSm, configured)) return rc;
+    return static_cast<int>(zb_launch(kernel, dim3(grid), dim3(32 * kWarps), grid > num_sms ? kRing : kOnePerSm, stream, p));
+  };
+  static bool one[16] = {}, two[16] = {};
+  if (const int rc = m <= 8 ? launch(zb_gemm_stream_kernel<1>, one) : launch(zb_gemm_stream_kernel<2>, two)) return rc;
   zb_count_launch(1);
-  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+  return static_cast<int>(cudaGetLastError());
 }
