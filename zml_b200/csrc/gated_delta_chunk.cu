@@ -440,42 +440,65 @@ __global__ void __launch_bounds__(2 * DVP) zb_gdn_scan_kernel(const GdnChunkPara
 }
 
 // ------------------------------------------------------------------------------------------
-// weight * y / rms(y) * silu(z), a warp per (token, head)
+// weight * y / rms(y) * silu(z): G lanes per (token, head), 16 bytes a lane, two of them on their way at once.  It should move three times
+// the outputs' bytes: 8192 tokens of 32 heads of 128, 201 MB, 30 us at the copy bandwidth; 60 us (86 with a warp per head, 8 bytes a
+// lane, one at a time and a division for every one).
+template <int G>
 __global__ void __launch_bounds__(256) zb_gdn_norm_kernel(const GdnChunkParams p) {
   zb_pdl_launch();
   zb_pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long long items = static_cast<long long>(p.tokens) * p.hv;
-  for (long long it = (blockIdx.x * 256ll + threadIdx.x) >> 5; it < items; it += gridDim.x * 8ll) {
-    const long long t = it / p.hv;
-    const int h = static_cast<int>(it - t * p.hv);
-    float f[2][4], ss = 0.f;
-    uint2 zr[2];
+  const int at = (threadIdx.x & (G - 1)) * 8;
+  const bool mine = at < p.dv;
+  float w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = mine ? __bfloat162float(p.norm_w[at + i]) : 0.f;
+  const long long first = (blockIdx.x * 256ll + threadIdx.x) / G, stride = gridDim.x * (256ll / G), items = static_cast<long long>(p.tokens) * p.hv;
+  const long long t_step = stride / p.hv;
+  const int h_step = static_cast<int>(stride - t_step * p.hv);
+  long long t = first / p.hv;
+  int h = static_cast<int>(first - t * p.hv);
+  const long long warp_first = (blockIdx.x * 256ll + (threadIdx.x & ~31)) / G;
+  for (long long base = warp_first; base < items; base += 2 * stride) {      // a warp goes through the loop as a whole
+    uint4 y[2], z[2];
+    long long to[2];
+    bool in[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int e = lane * 4 + k * 128;
-      if (e < p.dv) {
-        const uint2 u = *reinterpret_cast<const uint2*>(p.y + it * p.dv + e);
-        zr[k] = *reinterpret_cast<const uint2*>(p.z + t * p.ld_z + static_cast<long long>(h) * p.dv + e);
-        f[k][0] = lo_of(u.x);
-        f[k][1] = hi_of(u.x);
-        f[k][2] = lo_of(u.y);
-        f[k][3] = hi_of(u.y);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ss = fmaf(f[k][i], f[k][i], ss);
+      in[k] = mine && t < p.tokens;
+      y[k] = z[k] = make_uint4(0u, 0u, 0u, 0u);
+      const long long col = static_cast<long long>(h) * p.dv + at;
+      if (in[k]) {
+        y[k] = *reinterpret_cast<const uint4*>(p.y + t * p.hv * p.dv + col);
+        z[k] = *reinterpret_cast<const uint4*>(p.z + t * p.ld_z + col);
+      }
+      to[k] = t * p.ld_out + col;
+      t += t_step;
+      h += h_step;
+      if (h >= p.hv) {
+        h -= p.hv;
+        ++t;
       }
     }
-    const float inv = rsqrtf(zb_warp_sum(ss) / static_cast<float>(p.dv) + p.eps);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int e = lane * 4 + k * 128;
-      if (e < p.dv) {
-        const float z[4] = {lo_of(zr[k].x), hi_of(zr[k].x), lo_of(zr[k].y), hi_of(zr[k].y)};
-        float o[4];
+      const uint32_t yu[4] = {y[k].x, y[k].y, y[k].z, y[k].w}, zu[4] = {z[k].x, z[k].y, z[k].z, z[k].w};
+      float f[8], ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = f[k][i] * inv * __bfloat162float(p.norm_w[e + i]) * (z[i] / (1.f + __expf(-z[i])));
-        *reinterpret_cast<uint2*>(p.out + t * p.ld_out + static_cast<long long>(h) * p.dv + e) = make_uint2(zb_pack_bf16x2(o[0], o[1]), zb_pack_bf16x2(o[2], o[3]));
+      for (int i = 0; i < 4; ++i) {
+        f[2 * i] = lo_of(yu[i]);
+        f[2 * i + 1] = hi_of(yu[i]);
+        ss = fmaf(f[2 * i], f[2 * i], fmaf(f[2 * i + 1], f[2 * i + 1], ss));
       }
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = rsqrtf(ss / static_cast<float>(p.dv) + p.eps);
+      uint32_t o4[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float z0 = lo_of(zu[i]), z1 = hi_of(zu[i]);
+        o4[i] = zb_pack_bf16x2(f[2 * i] * inv * w[2 * i] * (z0 / (1.f + __expf(-z0))), f[2 * i + 1] * inv * w[2 * i + 1] * (z1 / (1.f + __expf(-z1))));
+      }
+      if (in[k]) *reinterpret_cast<uint4*>(p.out + to[k]) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
     }
   }
 }
@@ -498,8 +521,10 @@ int launch_chunked(const GdnChunkParams& p, cudaStream_t s) {
   zb_launch(zb_gdn_prep_kernel<DK>, dim3(static_cast<unsigned>((items + kPrepWarps - 1) / kPrepWarps)), dim3(32 * kPrepWarps), kSmem, s, p);
   if (const int rc = static_cast<int>(cudaGetLastError())) return rc;
   if (const int rc = p.dv % 64 == 0 ? launch_scan<DK, 64>(p, s) : launch_scan<DK, 32>(p, s)) return rc;
-  const long long warps = static_cast<long long>(p.tokens) * p.hv;
-  zb_launch(zb_gdn_norm_kernel, dim3(static_cast<unsigned>(std::min(148ll * 8, (warps + 7) / 8))), dim3(256), 0, s, p);
+  const int lanes = p.dv <= 32 ? 4 : (p.dv <= 64 ? 8 : (p.dv <= 128 ? 16 : 32));
+  const auto norm = lanes == 4 ? zb_gdn_norm_kernel<4> : (lanes == 8 ? zb_gdn_norm_kernel<8> : (lanes == 16 ? zb_gdn_norm_kernel<16> : zb_gdn_norm_kernel<32>));
+  const long long blocks = (static_cast<long long>(p.tokens) * p.hv * lanes + 255) / 256;
+  zb_launch(norm, dim3(static_cast<unsigned>(std::min(148ll * 8, blocks))), dim3(256), 0, s, p);
   zb_count_launch(3);
   return static_cast<int>(cudaGetLastError());
 }
