@@ -21,7 +21,7 @@
 // multiply-add per chunk outside the tensor core, whose additions truncate.
 //
 // What bounds it: mma.sync, of which one m16n8k16 takes a quarter of an SM about 32 clocks: a chunk of a warp is 168 of them and about
-// 900 other instructions, 2.9 us (5500 clocks), and the next chunk waits for it.  32 heads of 128: 4096 tokens of one sequence 0.75 ms
+// 900 other instructions, 2.9 us (5500 clocks), and the next chunk waits for it.  32 heads of 128: 4096 tokens of one sequence 0.48 ms
 // (the walk token by token: 8.1), 8192 tokens of 7 sequences of 128 .. 2048 0.55 (4.3), 8 x 512 0.24 (1.23).  Against 64 bits the
 // outputs are off as before (the bf16 rounding, 2.2e-3), the state by 0.4 - 1.3 times the walk's 7e-8 .. 1.5e-6.
 #include <cuda_bf16.h>
@@ -507,8 +507,14 @@ template <int DK, int DVP>
 int launch_scan(const GdnChunkParams& p, cudaStream_t s) {
   constexpr int kSmem = kStages * sizeof(ScanStage<DK, DVP>) + (DVP / 16) * kC * 24 * 2;
   static bool configured[16] = {};
-  if (const int rc = zb_config_smem_once(zb_gdn_scan_kernel<DK, DVP>, kSmem, configured)) return rc;
-  zb_launch(zb_gdn_scan_kernel<DK, DVP>, dim3(p.hv * (p.dv / DVP), p.num_seqs), dim3(2 * DVP), kSmem, s, p);
+  constexpr int kShare = 227 * 1024, kMost = kShare / 2 + 1024;
+  if (const int rc = zb_config_smem_once(zb_gdn_scan_kernel<DK, DVP>, std::max(kSmem, kMost), configured)) return rc;
+  // A CTA asks for so much shared memory that an SM holds no more of them than its part: those that start while zb_gdn_prep still holds
+  // most SMs would otherwise crowd on the others, where they share a tensor core for as long as they run: one sequence of 4096 tokens (64 CTAs)
+  // 0.72 - 0.80 ms so, 0.48 on an SM each; eight of 512 (512 CTAs) 0.234 either way.
+  const long long ctas = static_cast<long long>(p.hv) * (p.dv / DVP) * p.num_seqs, per_sm = (ctas + 147) / 148;
+  const int smem = std::max(kSmem, static_cast<int>(kShare / (per_sm + 1)) / 16 * 16 + 1024);
+  zb_launch(zb_gdn_scan_kernel<DK, DVP>, dim3(p.hv * (p.dv / DVP), p.num_seqs), dim3(2 * DVP), smem, s, p);
   return static_cast<int>(cudaGetLastError());
 }
 
