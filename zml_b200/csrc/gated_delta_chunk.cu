@@ -20,8 +20,8 @@
 // products of pieces.  The large products have an accumulator apart from the small ones, and the state is updated by one fused
 // multiply-add per chunk outside the tensor core, whose additions truncate.
 //
-// What bounds it: mma.sync, of which one m16n8k16 takes a quarter of an SM about 32 clocks: a chunk of a warp is 168 of them and about
-// 900 other instructions, 2.9 us (5500 clocks), and the next chunk waits for it.  32 heads of 128: 4096 tokens of one sequence 0.48 ms
+// What bounds it: mma.sync: a chunk of a warp is 168 of them and about 900 other instructions, 1.6 us (3100 clocks) with a quarter of an
+// SM to itself, and the next chunk waits for it.  (Q S on the FMA pipes instead: twice as long.)  32 heads of 128: 4096 tokens of one sequence 0.48 ms
 // (the walk token by token: 8.1), 8192 tokens of 7 sequences of 128 .. 2048 0.55 (4.3), 8 x 512 0.24 (1.23).  Against 64 bits the
 // outputs are off as before (the bf16 rounding, 2.2e-3), the state by 0.4 - 1.3 times the walk's 7e-8 .. 1.5e-6.
 #include <cuda_bf16.h>
