@@ -339,6 +339,31 @@ def test_paged_prefill_page_edges(hd, lens):
         expect_close(got.float(), want.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("junk", [float("nan"), float("inf"), 3e38])
+def test_paged_prefill_ignores_rows_behind_a_sequence(hd, junk):
+    """What a page holds behind the end of its sequence, and unused pages, do not reach the result: to the bit that of a clean cache."""
+    torch.manual_seed(hd)
+    hq, hkv, page = 4, 2, 64
+    parts = [(1, 0), (63, 0), (64, 64), (65, 63), (130, 70), (3, 700), (200, 120)]          # tokens, tokens in the cache
+    q_lens, seq_lens = [n for n, _ in parts], [n + c for n, c in parts]
+    kc, vc, bt = _make_paged(len(parts), seq_lens, hkv, hd, page)
+    used = torch.zeros(kc.shape[:2], dtype=torch.bool, device=DEV)
+    for i, n in enumerate(seq_lens):
+        t = torch.arange(n, device=DEV)
+        used[bt[i, t // page].long(), t % page] = True
+    q, qs = _randn(sum(q_lens), hq, hd), [0]
+    for n in q_lens:
+        qs.append(qs[-1] + n)
+    sl, qst = torch.tensor(seq_lens, dtype=torch.int32, device=DEV), torch.tensor(qs, dtype=torch.int32, device=DEV)
+    for window in (0, 100):
+        kc[~used], vc[~used] = 0.0, 0.0
+        clean = ops.paged_prefill(q, kc, vc, bt, sl, qst, window=window, impl="tc")
+        kc[~used], vc[~used] = junk, -junk
+        assert torch.equal(ops.paged_prefill(q, kc, vc, bt, sl, qst, window=window, impl="tc"), clean)
+        assert bool(clean.isfinite().all())
+
+
 @pytest.mark.parametrize("layout,rot", [(0, None), (1, None), (0, 32), (2, 32)])
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_rope_kvwrite(layout, rot, qk_norm):

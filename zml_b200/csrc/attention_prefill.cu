@@ -46,10 +46,10 @@ ZB_DEVICE float max_nan(float a, float b) {
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
   return d;
 }
-// 2^x of two numbers on the FMA pipes; x is cut at -126, a NaN stays one.
+// 2^x of two numbers on the FMA pipes; below -126.5 zero (as ex2.approx.ftz below -126), so that a masked key has no weight; a NaN stays one.
 ZB_DEVICE void exp2_fma(float& x0, float& x1) {
   const float kMagic = 12582912.f;                   // 1.5 * 2^23: the sum's low bits are x rounded to an integer
-  const ZbF2 x = zb_pack2(max_nan(x0, -126.f), max_nan(x1, -126.f)), t = zb_add2(x, zb_pack2(kMagic, kMagic));
+  const ZbF2 x = zb_pack2(max_nan(x0, -127.f), max_nan(x1, -127.f)), t = zb_add2(x, zb_pack2(kMagic, kMagic));
   const ZbF2 f = zb_fma2(zb_add2(t, zb_pack2(-kMagic, -kMagic)), zb_pack2(-1.f, -1.f), x);
   ZbF2 q = zb_pack2(kExp2[5], kExp2[5]);
 #pragma unroll
@@ -84,7 +84,7 @@ struct Shape {
   // Of 16 pairs of exponentials, those that the FMA pipes take.  8192 queries on 16384 keys, 32 heads: head_dim 64 0 / 4 / 6 / 8 pairs
   // 1246 / 1189 / 1270 / 1357 us, head_dim 128 0 / 1 / 4 1380 / 1352 / 1395 us.  More of them fill the ALU pipe (cuts, exponents).
   static constexpr int kPoly = HD == 64 ? 4 : 1;
-  static constexpr int kSmem = kHeads * kQBytes + 2 * kStages * kKvBytes + 1024 + 256;
+  static constexpr int kSmem = kHeads * kQBytes + 2 * kStages * kKvBytes + 1024 + 512;
 };
 constexpr uint32_t kColS = 0, kColO = 256;           // S: [head][buffer][64], O: [head][128] or [256]
 
@@ -115,7 +115,8 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* s_full = kv_empty + kStages;             // [2 heads][2 buffers]
   uint64_t* p_full = s_full + 4;                     // [2 heads][2 buffers], four warps
   uint64_t* o_ready = p_full + 4;                    // 2
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_ready + 2);
+  uint64_t* v_clean = o_ready + 2;                   // 1
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -149,6 +150,9 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int last_key = min(len, ctx + row_base + kRows);                                    // exclusive
   const int first_tile = p.window > 0 ? max(0, ctx + row_base - p.window + 1) / kKeys : 0;
   const int n_tiles = (last_key + kKeys - 1) / kKeys - first_tile;
+  // Rows of the last page behind the sequence's end.  They hold whatever was there before, perhaps NaN, and a masked key's weight of zero
+  // does not make that zero: these rows of V are cleared in shared memory (those of K only reach scores that the mask replaces).
+  const int behind = (first_tile + n_tiles) * kKeys - len;
 
   if (threadIdx.x == 0) {
     zb_mbar_init(q_full, 1);
@@ -163,6 +167,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     zb_mbar_init(&o_ready[0], 1);
     zb_mbar_init(&o_ready[1], 1);
+    zb_mbar_init(v_clean, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -182,6 +187,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   if (warp == 4 * kHeads) {
     // ------------------------------------------------------------------ TMA producer
+    bool ok = true;
     if (lane == 0) {
       const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
       zb_mbar_expect_tx(q_full, kHeads * S::kQBytes);
@@ -192,6 +198,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       for (int j = 0; j < n_tiles; ++j) {
         if (j >= kStages && !zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag)) {
           *abort_where = 1u;
+          ok = false;
           break;
         }
         int page = bt[first_tile + j];
@@ -204,6 +211,20 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           stage = 0;
           phase ^= 1u;
         }
+      }
+    }
+    if (n_tiles > 0 && behind > 0 && __all_sync(0xffffffffu, ok)) {
+      const int last = n_tiles - 1, at = last % kStages;
+      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / kStages) & 1u, abort_flag);
+      if (__all_sync(0xffffffffu, ok)) {
+        uint4* v = reinterpret_cast<uint4*>(v_s + at * S::kKvBytes) + (kKeys - behind) * 8;      // the swizzle stays within a row of 128 bytes
+        for (int c = 0; c < S::kSubs; ++c)
+          for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+        zb_fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) zb_mbar_arrive(v_clean);
+      } else {
+        *abort_where = 7u;
       }
     }
   } else if (warp > 4 * kHeads) {
@@ -239,7 +260,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         where = 3u;
       }
       for (int j = 0; where == 0u && j < n_tiles; ++j) {
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == n_tiles - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
           where = 4u;
           break;
         }
