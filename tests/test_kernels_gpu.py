@@ -158,6 +158,29 @@ def test_gemm_pair_tiles(m, n, k):
         b.zero_()
 
 
+@pytest.mark.parametrize("m,n", [(3, 264), (40, 264), (70, 264), (70, 4104), (128, 264), (200, 136), (200, 264), (300, 264), (300, 136), (600, 520)])
+def test_gemm_unaligned_output(m, n):
+    """Outputs and residuals whose rows do not start on 16 bytes: float32 rows of an odd stride, views that begin 4 bytes into a buffer;
+    what lies around them stays as it was."""
+    torch.manual_seed(m + n)
+    k = 320
+    a, w, bias = _randn(m, k), _randn(n, k, scale=1.0 / math.sqrt(k)), _randn(n)
+    base = a.float() @ w.float().t() + bias.float()
+    buf = torch.full((m, n + 3), 7.0, device=DEV)
+    expect_close(ops.gemm(a, w, bias=bias, out=buf[:, 1:n + 1]), base, atol=1e-4, rtol=1e-4, min_close=ALL)
+    assert bool((buf[:, 0] == 7).all() and (buf[:, n + 1:] == 7).all())
+    flat, rflat = torch.full((m * (n + 8) + 8,), 7.0, dtype=torch.bfloat16, device=DEV), _randn(m * (n + 8) + 8)
+    out, res = (f[2:2 + m * (n + 8)].view(m, n + 8)[:, :n] for f in (flat, rflat))
+    want = base + res.float()
+    expect_close(ops.gemm(a, w, bias=bias, residual=res, out=out).float(), want, atol=3e-2, rtol=2e-2, min_close=ALL)
+    assert bool((flat[:2] == 7).all() and (flat[2:2 + m * (n + 8)].view(m, n + 8)[:, n:] == 7).all())
+    expect_close(ops.gemm(a, w, bias=bias, residual=res, out=res).float(), want, atol=3e-2, rtol=2e-2, min_close=ALL)
+    act = flat[2:2 + m * (n + 8)].view(m, n + 8)[:, :n // 2]
+    gu = a.float() @ w.float().t()
+    expect_close(ops.gemm(a, ops.interleave_gate_up(w), out=act, swiglu=True).float(), torch.nn.functional.silu(gu[:, :n // 2]) * gu[:, n // 2:], atol=3e-2, rtol=2e-2,
+                 min_close=ALL)
+
+
 @pytest.mark.parametrize("rows,d", [(1, 2048), (33, 4096), (64, 8192), (5, 1024 + 8), (3, 16384)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm(rows, d, with_res):

@@ -55,6 +55,7 @@ struct Gemm2Params {
   const __nv_bfloat16* bias;
   int out_f32;
   int static_w;                 // W may be read before the kernel in front is done
+  int rows16;                   // rows of out and residual start on 16 bytes
   int num_m, num_n;             // tiles of 256 x BN
   int group_m;                  // rasterisation: tiles of `group_m` consecutive row blocks share their W tiles in L2
   ZbGemmEpi epi;                // all but pf_*; out_sumsq has a part per tile column
@@ -281,7 +282,7 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * row_scale;
-        const bool whole = q + 32 <= prm.n;
+        const bool whole = prm.rows16 && q + 32 <= prm.n;      // else element by element
         if (prm.bias != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
@@ -452,6 +453,7 @@ int zb_gemm_2cta_launch(const void* a, const void* w, void* out, const void* res
   prm.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   prm.out_f32 = out_f32 & 1;
   prm.static_w = static_w;
+  prm.rows16 = zb_gemm_rows16(out, residual, ldo, prm.out_f32);
   prm.group_m = 8;
   if (epi != nullptr) prm.epi = *epi;
   prm.status = status;

@@ -53,7 +53,7 @@ struct GemmParams {
   int units_per_cta; // k-blocks per CTA (stream-K range length)
   int rr_tiles;      // > 0: whole tiles dealt round-robin, this many per CTA (large problems)
   int group_p;       // rasterisation group height (P tiles)
-  int flags;         // bit 0: the weight operand is not written by the preceding kernel
+  int flags;         // bit 0: the weight operand is not written by the preceding kernel; bit 1: rows of out and residual start on 16 bytes
   int l2_prefetch;   // weight tiles per CTA to pull into L2 ahead of the shared-memory ring
   int cluster;       // > 1: the CTAs of a cluster split one tile along K and reduce it through shared memory
   unsigned long long* timeline;   // optional [grid][8] globaltimer stamps of this launch's phases (profiling)
@@ -947,6 +947,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
         }
       };
       // bias / residual (read from this rank's memory) then store into `outp`
+      const bool rows16 = (prm.flags & 2) != 0;
       auto finish_chunk = [&](int c0, float (&v)[16]) {
         if constexpr (SWAP) {
           const float b = (prm.bias && p < prm.rows_p) ? __bfloat162float(prm.bias[p]) : 0.f;
@@ -964,7 +965,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           const size_t o = static_cast<size_t>(p) * prm.ldo + q;
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] *= row_scale;
-          if (q + 16 <= prm.rows_q) {
+          if (rows16 && q + 16 <= prm.rows_q) {
             if (prm.bias) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) v[j] += __bfloat162float(prm.bias[q + j]);
@@ -1007,7 +1008,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           // p = output row m, q = output column n (16 consecutive columns per step)
           const int q = q0 + c0;
           const size_t o = static_cast<size_t>(p) * prm.ldo + q;
-          if (q + 16 <= prm.rows_q) {
+          if (rows16 && q + 16 <= prm.rows_q) {
             if (prm.out_f32) {
               float4* op = reinterpret_cast<float4*>(reinterpret_cast<float*>(outp) + o);
 #pragma unroll
@@ -1048,7 +1049,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           const int q = q0 + c0;
           if (p < prm.rows_p) {
             const size_t o = static_cast<size_t>(p) * prm.ldo + (q >> 1);
-            if (q + 16 <= prm.rows_q) {
+            if (rows16 && q + 16 <= prm.rows_q) {
               uint32_t w[4];
 #pragma unroll
               for (int j = 0; j < 4; ++j)
@@ -1123,7 +1124,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
 #pragma unroll
             for (int e = 0; e < 4; ++e) bz[e] = (pb + e) < prm.rows_p ? __bfloat162float(prm.bias[pb + e]) : 0.f;
           }
-          const bool vec = (pb + 3) < prm.rows_p && (prm.ldo % 4) == 0;
+          const bool vec = (pb + 3) < prm.rows_p && rows16;
           // residual loads first, all of them: `out` may alias `residual`, which would otherwise
           // order every load behind the previous column's store
           uint2 rres[kCols];
@@ -1736,7 +1737,7 @@ namespace {
 
 int launch_row_sumsq(const void* x, int rows, int d, long long ld, float* out, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if ((d % 8) != 0 || (ld % 8) != 0) return -10;
+  if ((d % 8) != 0 || (ld % 8) != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return -10;
   const cudaError_t e = zb_launch(zb_row_sumsq_kernel, dim3(static_cast<unsigned>(rows)), dim3(256), 0, stream,
                                   reinterpret_cast<const __nv_bfloat16*>(x), ld, d, out);
   zb_count_launch(1);
@@ -1819,7 +1820,7 @@ int gemm_impl(const void* a, const void* w, void* out, const void* residual, con
   prm.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   prm.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   prm.out_f32 = out_f32;
-  prm.flags = static_w;
+  prm.flags = static_w | (zb_gemm_rows16(out, residual, ldo, out_f32) ? 2 : 0);
   prm.l2_prefetch = l2_prefetch_tiles(sw, bn, grid, rr);
   prm.timeline = next_timeline(grid);
   prm.group_p = (band != nullptr && band->mode != 0) ? 8 : 16;     // band pipeline: bands finish (and start) in groups of 8
@@ -2076,7 +2077,7 @@ int zb_gemm_ar_fused_epi(const ZbArContext* ctx, const void* a, const void* w, s
   prm.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   prm.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   prm.out_f32 = 0;
-  prm.flags = 1;     // `w` is a model parameter in every use of the fused kernel
+  prm.flags = 3;     // `w` is a model parameter in every use of the fused kernel, the buffers start on 16 bytes
   prm.l2_prefetch = l2_prefetch_tiles(sw, bn, grid, rr);
   prm.timeline = next_timeline(grid);
   prm.group_p = 16;

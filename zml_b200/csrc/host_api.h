@@ -40,6 +40,12 @@ struct ZbArContext {
   void* mc_heap;          // NVLink multicast address of the heaps (one address, every rank's copy), or null
 };
 
+// Whether the rows of a GEMM's output (fp32 or bf16) and of its bf16 residual, both with leading dimension `ldo`, start on 16 bytes: where
+// they do not, the epilogues go element by element.
+inline bool zb_gemm_rows16(const void* out, const void* residual, int ldo, int out_f32) {
+  return ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 15) == 0 && (ldo & (out_f32 && residual == nullptr ? 3 : 7)) == 0;
+}
+
 // Optional epilogue work of the bf16 GEMM (gemm_bf16.cu).  All pointers are local device memory.
 //   in_sumsq : partial sums of squares of the activation rows, [in_parts][in_ld] fp32; the accumulator of
 //              token t is multiplied by rsqrt(sum_i in_sumsq[i][t] * in_inv_d + in_eps) before bias and
