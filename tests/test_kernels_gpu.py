@@ -387,6 +387,29 @@ def test_paged_prefill_ignores_rows_behind_a_sequence(hd, junk):
         assert bool(clean.isfinite().all())
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+def test_paged_prefill_alignment(hd):
+    """An `out` that does not start on 16 bytes goes to the kernel that stores 4 at a time; inputs that do not are refused."""
+    torch.manual_seed(hd)
+    seq_lens, qs = [70, 130], [0, 70, 200]
+    kc, vc, bt = _make_paged(2, seq_lens, 2, hd, 64)
+    sl, qst = torch.tensor(seq_lens, dtype=torch.int32, device=DEV), torch.tensor(qs, dtype=torch.int32, device=DEV)
+    q = _randn(200, 4, hd)
+    want = ref.paged_attention(q, kc, vc, bt, seq_lens, qs)
+    flat = torch.zeros(q.numel() + 8, dtype=torch.bfloat16, device=DEV)
+    out = flat[4:4 + q.numel()].view(q.shape)
+    expect_close(ops.paged_prefill(q, kc, vc, bt, sl, qst, out=out).float(), want.float(), atol=2e-2, rtol=2e-2, min_close=ALL)
+    assert not flat[:4].any() and not flat[4 + q.numel():].any()
+
+    def moved(t):
+        return torch.zeros(t.numel() + 8, dtype=t.dtype, device=DEV)[4:4 + t.numel()].view(t.shape)
+    for args in ((moved(q), kc, vc), (q, moved(kc), vc), (q, kc, moved(vc))):
+        with pytest.raises(ValueError):
+            ops.paged_prefill(*args, bt, sl, qst)
+    with pytest.raises(ValueError):
+        ops.paged_prefill(q, kc, vc, bt, sl, qst, out=out, impl="tc")
+
+
 @pytest.mark.parametrize("layout,rot", [(0, None), (1, None), (0, 32), (2, 32)])
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_rope_kvwrite(layout, rot, qk_norm):

@@ -633,6 +633,7 @@ int zb_paged_prefill_tc(const void* q, const void* k_cache, const void* v_cache,
   if (!zb_paged_prefill_tc_supported(num_q_heads, num_kv_heads, head_dim, kKeys) || (ext != nullptr && head_dim != kHD)) return -32;
   ZbDeviceState* st = zb_device_state();
   if (!st) return -20;
+  if (ext == nullptr && (reinterpret_cast<uintptr_t>(out) & 15) != 0) return -33;
   total_q_blocks128 = std::min(total_q_blocks128, total_tokens / kQRows + batch);      // a caller may count blocks of 64 rows
   if (ext == nullptr)
     return zb_prefill_plain(q, k_cache, v_cache, out, block_table, seq_lens, q_start, batch, total_q_blocks128, total_tokens, num_q_heads,

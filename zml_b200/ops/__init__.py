@@ -398,8 +398,6 @@ _ATTN_TC = _os.environ.get("ZB_ATTN_TC", "1") != "0"
 def _tc_takes(q, k_cache, ext) -> bool:
     l = _lib.lib()
     ok = bool(l.zb_paged_prefill_tc_supported(q.shape[1], k_cache.shape[2], q.shape[2], k_cache.shape[1])) and q.stride(0) % 8 == 0
-    if q.shape[2] != 128 and ext is None:           # tensor maps start on 16 bytes; the mma.sync kernel takes other pointers
-        return ok and (q.data_ptr() | k_cache.data_ptr()) % 16 == 0
     return ok and (ext is None or (q.shape[2] == 128 and bool(l.zb_paged_prefill_tc_ext_supported(ext.cap, ext.pair))))
 
 
@@ -428,9 +426,12 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
     assert q_start.dtype == torch.int32 and block_table.is_contiguous()
     if out is None:
         out = torch.empty((t, hq, hd), dtype=q.dtype, device=q.device)
+    if (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 or q.stride(0) % 8 or (ext is None and out.data_ptr() % 4):
+        raise ValueError("prefill attention copies 16 bytes at a time: rows of q and the caches start on 16 bytes, those of out on 4")
     nqb = total_q_blocks if total_q_blocks is not None else t // 64 + b
     l = _lib.lib()
-    tc_ok = _tc_takes(q, k_cache, ext)
+    # the tcgen05 kernel stores rows of 16-byte pieces; the other one stores 4 bytes at a time
+    tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or out.data_ptr() % 16 == 0)
     if impl == "tc" and not tc_ok:
         raise ValueError(f"the tensor-core prefill kernel does not take hq={hq} hkv={hkv} hd={hd} page={page}")
     if tc_ok and (impl == "tc" or (impl == "auto" and _ATTN_TC)):
