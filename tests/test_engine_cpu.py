@@ -389,6 +389,15 @@ def test_engine_rejects_bad_requests_without_stranding_pages():
     assert eng.generate([[1, 2, 3]], 0)[0] == [[]]
 
 
+def test_a_step_without_entries_returns_nothing():
+    model = LlamaModel(LlamaConfig.from_hf(PRESETS["tiny-llama-test"])).init_random(seed=1)
+    eng = Engine(model, num_pages=8, page_size=16, max_batch=2, max_seq_len=64)
+    assert eng.step([]) is None and eng.step([], []) is None
+    r = eng.open_request()
+    eng.step([(r, [1, 2, 3])])
+    assert eng.step([(r, [4])]) is None and eng.step([(r, [5])], [[0]]).shape == (1, model.config.vocab_size)
+
+
 def test_serve_reports_tokens_block_by_block():
     """`on_tokens` sees every token exactly once, in order, per prompt, and one final call per prompt."""
     cfg = LlamaConfig.from_hf(dict(PRESETS["tiny-llama-test"], vocab_size=300))

@@ -310,7 +310,7 @@ class Engine:
         if all(b - a == 1 and a > 0 for _, a, b in chunk) and len(chunk) <= self.max_batch:
             lg = self._step_decode(chunk)
             rows = [i for i, w in enumerate(want) for _ in w]
-            if rows == list(range(lg.shape[0])):
+            if rows and rows == list(range(lg.shape[0])):
                 lg = lg.clone()                  # the capture's buffer is written again by the next step
             elif rows:
                 at = self._host(len(rows))
