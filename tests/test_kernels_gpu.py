@@ -388,6 +388,18 @@ def test_paged_prefill_ignores_rows_behind_a_sequence(hd, junk):
 
 
 @pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("scale", [-0.2, 0.0])
+def test_paged_prefill_scale_below_zero(hd, scale):
+    torch.manual_seed(hd)
+    seq_lens, qs = [70, 200], [0, 70, 200]
+    kc, vc, bt = _make_paged(2, seq_lens, 2, hd, 64)
+    sl, qst = torch.tensor(seq_lens, dtype=torch.int32, device=DEV), torch.tensor(qs, dtype=torch.int32, device=DEV)
+    q = _randn(200, 4, hd)
+    want = ref.paged_attention(q, kc, vc, bt, seq_lens, qs, scale)
+    expect_close(ops.paged_prefill(q, kc, vc, bt, sl, qst, scale).float(), want.float(), atol=2e-2, rtol=2e-2, min_close=ALL)
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
 def test_paged_prefill_alignment(hd):
     """An `out` that does not start on 16 bytes goes to the kernel that stores 4 at a time; inputs that do not are refused."""
     torch.manual_seed(hd)

@@ -430,21 +430,22 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
         raise ValueError("prefill attention copies 16 bytes at a time: rows of q and the caches start on 16 bytes, those of out on 4")
     nqb = total_q_blocks if total_q_blocks is not None else t // 64 + b
     l = _lib.lib()
-    # the tcgen05 kernel stores rows of 16-byte pieces; the other one stores 4 bytes at a time
-    tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or out.data_ptr() % 16 == 0)
+    scale = float(scale if scale is not None else 1.0 / math.sqrt(hd))
+    # the tcgen05 kernel stores rows of 16-byte pieces and scales the row's maximum (no larger any more with a scale below zero) and the mask;
+    # the other one stores 4 bytes at a time and takes the maximum of the scaled scores
+    tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or (out.data_ptr() % 16 == 0 and scale > 0))
     if impl == "tc" and not tc_ok:
         raise ValueError(f"the tensor-core prefill kernel does not take hq={hq} hkv={hkv} hd={hd} page={page}")
     if tc_ok and (impl == "tc" or (impl == "auto" and _ATTN_TC)):
         rc = l.zb_paged_prefill_tc(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _ptr(seq_lens), _ptr(q_start), b, nqb, t,
-            hq, hkv, hd, block_table.shape[1], q.stride(0), float(scale if scale is not None else 1.0 / math.sqrt(hd)), int(window),
+            hq, hkv, hd, block_table.shape[1], q.stride(0), scale, int(window),
             int(_os.environ.get("ZB_ATTN_V_LBO", "0")), int(_os.environ.get("ZB_ATTN_V_SBO", "0")), _ext(ext), _lib.stream_ptr())
         _lib.check(rc, "zb_paged_prefill_tc")
         return out
     rc = _lib.lib().zb_paged_prefill(
         _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _ptr(seq_lens),
-        _ptr(q_start), b, nqb, hq, hkv, hd, page, block_table.shape[1], q.stride(0),
-        float(scale if scale is not None else 1.0 / math.sqrt(hd)), int(window), _ext(ext), _lib.stream_ptr())
+        _ptr(q_start), b, nqb, hq, hkv, hd, page, block_table.shape[1], q.stride(0), scale, int(window), _ext(ext), _lib.stream_ptr())
     _lib.check(rc, "zb_paged_prefill")
     return out
 
