@@ -119,6 +119,22 @@ def test_causal_conv1d_token_blocks(k, c):
     assert torch.equal(st_gpu.cpu(), st_cpu)
 
 
+@pytest.mark.parametrize("k,c,lens", [(3, 1032, [4800, 37, 2]), (4, 64, [16, 3, 15]), (2, 8, [1, 2, 1, 17])])
+def test_causal_conv1d_routes(k, c, lens):
+    """Walked or cut along the tokens, into blocks of 4 to 32: the same bits, gates and caches included."""
+    torch.manual_seed(c)
+    qs, sl, _ = _seq_meta(lens, [5] * len(lens))
+    slots = torch.arange(len(lens), dtype=torch.int32)
+    x, pre, post = (torch.randn(sum(lens), c).bfloat16().to(DEV) for _ in range(3))
+    w, st = (torch.randn(c, k) * 0.5).bfloat16().to(DEV), torch.randn(len(lens), k - 1, c).bfloat16().to(DEV)
+    res = []
+    for longest in (1, max(lens, default=0) + 15, None):
+        s = st.clone()
+        res.append((la.causal_conv1d(x, w, s, qs.to(DEV), sl.to(DEV), slots.to(DEV), pre=pre, post=post, silu=True, longest=longest), s))
+    for out, s in res[1:]:
+        assert torch.equal(out, res[0][0]) and torch.equal(s, res[0][1])
+
+
 def test_sigmoid_gate_mul():
     buf = torch.randn(37, 256 + 128, device=DEV).bfloat16()
     x = buf[:, :128].clone()

@@ -12,8 +12,8 @@
 // The reference expresses the recurrence as a `stablehlo.while` over tokens (zml/nn.zig:1749-1874)
 // and the convolutions as XLA conv1d + scatter on a cache tensor
 // (examples/llm/models/qwen3_5/model.zig:882-980, examples/llm/models/lfm2/model.zig:441-500).
-// Here a sequence is walked once by one CTA per (sequence, head) or (sequence, channel block);
-// prefill chunks and decode steps use the same kernels, the state lives in a slot pool.
+// Here decode steps and short portions are walked token by token, by one CTA per (sequence, head) or (sequence, channel block); prompts are
+// cut along their tokens, the convolution below, the recurrence in gated_delta_chunk.cu.  The state lives in a slot pool.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -77,12 +77,9 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_kernel(const ConvParams 
   for (int j = 0; j < K - 1; ++j) st[static_cast<size_t>(j) * p.channels] = __float2bfloat16(win[j]);
 }
 
-// The same for rows that start on 16 bytes: a thread has eight channels and walks kConvTokens tokens of one sequence, so a prompt is cut
-// along its tokens as well (8192 channels, 8192 tokens of 7 sequences: the walk of a whole sequence above took 1214 us, bound by
-// the latency of one load per token; 141 us).  The inputs in front of a block are read again.  The block at a sequence's start owns
-// its cache: it reads it before it writes the sequence's last inputs to it.
-constexpr int kConvTokens = 32;
-
+// The same for rows that start on 16 bytes: a thread has eight channels and walks `per` tokens of one sequence, so a prompt is cut along
+// its tokens as well (the walk of a whole sequence above is bound by the latency of one load per token).  The inputs in front of a block
+// are read again.  The block at a sequence's start owns its cache: it reads it before it writes the sequence's last inputs to it.
 ZB_DEVICE void conv_unpack8(const uint4& u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -98,18 +95,19 @@ ZB_DEVICE uint4 conv_pack8(const float (&f)[8]) {
 ZB_DEVICE float conv_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
 template <int K>
-__global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const ConvParams p, int num_seqs) {
+__global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const ConvParams p, int num_seqs, int per) {
   zb_pdl_launch();
   zb_pdl_wait();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 8, cid = blockIdx.y;
-  // Sequence s has the blocks from q_start[s] / kConvTokens + s on, which are no fewer than it needs.
-  int s = 0;
-  for (int hi = num_seqs; hi - s > 1;) {
-    const int mid = (s + hi) >> 1;
-    if (p.q_start[mid] / kConvTokens + mid <= cid) s = mid; else hi = mid;
-  }
-  const int t0 = p.q_start[s], t1 = p.q_start[s + 1], a = t0 + (cid - (t0 / kConvTokens + s)) * kConvTokens, b = min(a + kConvTokens, t1);
-  if (c >= p.channels || a >= t1) return;
+  // Sequence s has the blocks from q_start[s] / per + s on, which are no fewer than it needs.  Every warp counts the sequences that begin at
+  // or in front of this block, a lane each.
+  int s = -1;
+#pragma unroll 4
+  for (int i = threadIdx.x & 31; i - (threadIdx.x & 31) < num_seqs; i += 32)
+    s += __popc(__ballot_sync(0xffffffffu, i < num_seqs && p.q_start[min(i, num_seqs)] / per + i <= cid));
+  if (c >= p.channels || s < 0) return;              // s < 0: rows in front of the first sequence
+  const int t0 = p.q_start[s], t1 = p.q_start[s + 1], a = t0 + (cid - (t0 / per + s)) * per, b = min(a + per, t1);
+  if (a >= t1) return;
   const bool fresh = p.seq_lens[s] - (t1 - t0) <= 0;
   if (!ZB_BC_OK(p.slots[s], ZB_BC_STATE_SLOTS, kKernelCausalConv, 2)) return;
   __nv_bfloat16* st = p.state + static_cast<size_t>(p.slots[s]) * (K - 1) * p.channels + c;
@@ -122,22 +120,22 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const Conv
       for (int i = 0; i < 8; ++i) x[i] = conv_round(x[i] * g[i]);
     }
   };
+  auto cached = [&](int j) { return fresh ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4*>(st + static_cast<size_t>(j) * p.channels); };
   float w[K][8], win[K - 1][8];
+  {
+    float taps[K][8];                                // 8 K taps of eight channels, in the order of memory
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int j = 0; j < K; ++j) conv_unpack8(reinterpret_cast<const uint4*>(p.w + static_cast<size_t>(c) * K)[j], taps[j]);
 #pragma unroll
-    for (int j = 0; j < K; ++j) w[j][i] = __bfloat162float(p.w[static_cast<size_t>(c + i) * K + j]);
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < K; ++j) w[j][i] = taps[(i * K + j) / 8][(i * K + j) % 8];
+  }
 #pragma unroll
   for (int j = 0; j < K - 1; ++j) {                  // the inputs of tokens a - (K - 1) + j
     const int t = a - (K - 1) + j;
-    if (t >= t0) {
-      input(t, win[j]);
-    } else if (!fresh) {
-      conv_unpack8(*reinterpret_cast<const uint4*>(st + static_cast<size_t>(t - t0 + K - 1) * p.channels), win[j]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) win[j][i] = 0.f;
-    }
+    if (t >= t0) input(t, win[j]);
+    else conv_unpack8(cached(t - t0 + K - 1), win[j]);
   }
   if (a == t0) {
     // the sequence's last K - 1 inputs, those in front of its first token among them
@@ -145,18 +143,13 @@ __global__ void __launch_bounds__(128) zb_causal_conv1d_blocks_kernel(const Conv
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) {
       const int t = t1 - (K - 1) + j;
-      float x[8];
       if (t >= t0) {
+        float x[8];
         input(t, x);
+        last[j] = conv_pack8(x);
       } else {
-#pragma unroll
-        for (int q = 0; q < K - 1; ++q)
-          if (q == t - t0 + K - 1) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = win[q][i];
-          }
+        last[j] = cached(t - t0 + K - 1);
       }
-      last[j] = conv_pack8(x);
     }
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) *reinterpret_cast<uint4*>(st + static_cast<size_t>(j) * p.channels) = last[j];
@@ -478,15 +471,20 @@ int launch_gdn(const GdnParams& p, int num_seqs, cudaStream_t s) {
   return static_cast<int>(cudaGetLastError());
 }
 
+// New tokens of the longest sequence from which a batch of prompts goes by blocks.  8192 channels, us, walk / blocks: 8 tokens 5.1 / 7.3,
+// 15 7.3 / 7.4, 16 7.6 / 7.3, 40 14.7 / 7.7, 200 62 / 8.1, 2000 599 / 34; 32 x 5 tokens 7.0 / 8.6.
+constexpr int kConvLong = 16;
+
 }  // namespace
 
 extern "C" {
 
-// Depthwise causal conv over a flattened varlen batch of `tokens` rows; `kernel_size` taps per channel, 2..5.
+// Depthwise causal conv over a flattened varlen batch of `tokens` rows; `kernel_size` taps per channel, 2..5.  `longest`: rows of the longest
+// sequence, an estimate that only chooses the kernel.
 int zb_causal_conv1d(const void* x, long long ldx, const void* pre, long long ldpre, const void* post,
                      long long ldpost, const void* w, void* out, long long ldo, void* state,
                      const int32_t* q_start, const int32_t* seq_lens, const int32_t* slots, int num_seqs,
-                     int tokens, int channels, int kernel_size, int silu, void* stream) {
+                     int tokens, int longest, int channels, int kernel_size, int silu, void* stream) {
   if (num_seqs <= 0 || channels <= 0) return 0;
   ConvParams p;
   p.x = reinterpret_cast<const __nv_bfloat16*>(x);
@@ -506,14 +504,17 @@ int zb_causal_conv1d(const void* x, long long ldx, const void* pre, long long ld
   p.silu = silu;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const auto at16 = [](const void* q, long long ld) { return q == nullptr || ((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld & 7) == 0); };
-  if (out != x && out != pre && channels % 8 == 0 && at16(x, ldx) && at16(pre, ldpre) && at16(post, ldpost) && at16(out, ldo) && at16(state, 0) &&
-      tokens / kConvTokens + num_seqs <= 65535) {
-    const dim3 blocks((channels / 8 + 127) / 128, tokens / kConvTokens + num_seqs);
+  if (longest >= kConvLong && out != x && out != pre && channels % 8 == 0 && at16(x, ldx) && at16(pre, ldpre) && at16(post, ldpost) &&
+      at16(out, ldo) && at16(state, 0) && at16(w, 0) && tokens / 32 + num_seqs <= 65535) {
+    const int columns = (channels / 8 + 127) / 128;
+    int per = 32;                                    // fewer tokens a block where there would not be two CTAs for every SM
+    while (per > 4 && columns * (tokens / per) < 2 * zb_num_sms() && tokens / (per / 2) + num_seqs <= 65535) per >>= 1;
+    const dim3 blocks(columns, tokens / per + num_seqs);
     switch (kernel_size) {
-      case 2: zb_launch(zb_causal_conv1d_blocks_kernel<2>, blocks, dim3(128), 0, s, p, num_seqs); break;
-      case 3: zb_launch(zb_causal_conv1d_blocks_kernel<3>, blocks, dim3(128), 0, s, p, num_seqs); break;
-      case 4: zb_launch(zb_causal_conv1d_blocks_kernel<4>, blocks, dim3(128), 0, s, p, num_seqs); break;
-      case 5: zb_launch(zb_causal_conv1d_blocks_kernel<5>, blocks, dim3(128), 0, s, p, num_seqs); break;
+      case 2: zb_launch(zb_causal_conv1d_blocks_kernel<2>, blocks, dim3(128), 0, s, p, num_seqs, per); break;
+      case 3: zb_launch(zb_causal_conv1d_blocks_kernel<3>, blocks, dim3(128), 0, s, p, num_seqs, per); break;
+      case 4: zb_launch(zb_causal_conv1d_blocks_kernel<4>, blocks, dim3(128), 0, s, p, num_seqs, per); break;
+      case 5: zb_launch(zb_causal_conv1d_blocks_kernel<5>, blocks, dim3(128), 0, s, p, num_seqs, per); break;
       default: return -70;
     }
     zb_count_launch(1);

@@ -32,6 +32,7 @@ class AttnMeta:
     state_slots: Optional[torch.Tensor] = None    # {b} slot of every sequence in a model's recurrent-state pool
     q_start_host: Optional[list] = None           # host copy of q_start (prefill), for splitting a chunk by sequences
     seq_lens_host: Optional[list] = None          # host copy of seq_lens (prefill)
+    max_q_len: Optional[int] = None               # new tokens of the longest sequence (prefill)
     plans: dict = field(default_factory=dict)     # what the layers derive from this step's metadata once (by their own keys)
 
 

@@ -231,7 +231,8 @@ class Lfm2Model(LlamaModel):
             q_start = torch.arange(n1.shape[0] + 1, dtype=torch.int32, device=n1.device)
         bcx = ops.gemm(n1, e["in_proj"], static_w=True)                # [T, B | C | x]
         return la.causal_conv1d(bcx[:, 2 * cl:3 * cl], e["conv_w"], self.conv_state[self.conv_index[l]], q_start,
-                                meta.seq_lens, meta.state_slots, pre=bcx[:, :cl], post=bcx[:, cl:2 * cl])
+                                meta.seq_lens, meta.state_slots, pre=bcx[:, :cl], post=bcx[:, cl:2 * cl],
+                                longest=meta.max_q_len)
 
     def layer(self, l: int, x, meta: AttnMeta, kv_cache):
         lw, c = self.layers[l], self.config

@@ -399,7 +399,7 @@ class Qwen35Model(LlamaModel):
         q_start, seq_lens, slots = self._seq_meta(meta, n1.shape[0])
         proj = ops.gemm(n1, w.in_proj, static_w=True)                   # [T, q|k|v|z|b|a]
         mix = la.causal_conv1d(proj[:, :self.conv_dim_l], w.conv_w, self.conv_state[i], q_start, seq_lens, slots,
-                               silu=True)
+                               silu=True, longest=meta.max_q_len)
         return la.gated_delta_scan(mix, proj[:, self.off_z:self.off_b], proj[:, self.off_a:self.off_a + self.hv_l],
                                    proj[:, self.off_b:self.off_a], w.a_log, w.dt_bias, w.norm_w, c.rms_norm_eps,
                                    self.rec_state[i], q_start, seq_lens, slots, self.hk_l, self.hv_l, self.dk, self.dv)

@@ -25,7 +25,7 @@ from . import _lib
 
 _p, _i, _ll, _f = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 _lib.register_signature("zb_causal_conv1d", _i, [_p, _ll, _p, _ll, _p, _ll, _p, _p, _ll, _p, _p, _p, _p, _i, _i,
-                                                _i, _i, _i, _p])
+                                                _i, _i, _i, _i, _p])
 _lib.register_signature("zb_gated_delta_scan", _i, [_p, _ll, _p, _ll, _p, _p, _ll, _p, _p, _p, _f, _p, _p, _ll,
                                                    _p, _p, _p, _i, _i, _i, _i, _i, _p])
 _lib.register_signature("zb_gated_delta_rec_bytes", C.c_size_t, [_i, _i, _i])
@@ -40,6 +40,11 @@ def _ptr(t: Optional[torch.Tensor]):
 
 def _bf16_round(x: torch.Tensor) -> torch.Tensor:
     return x.to(torch.bfloat16).float()
+
+
+def _longest(tokens: int, seq_lens: torch.Tensor, longest: Optional[int]) -> int:
+    """`longest`, or the most that one of these sequences can have."""
+    return longest if longest is not None else tokens - seq_lens.shape[0] + 1
 
 
 # ---------------------------------------------------------------------------- conv
@@ -69,9 +74,11 @@ def causal_conv1d_reference(x, w, state, q_start, seq_lens, slots, pre=None, pos
     return out
 
 
-def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, silu: bool = False, out=None):
+def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, silu: bool = False, out=None,
+                  longest: Optional[int] = None):
     """x [T, C] (row stride free), w [C, K] taps (tap K-1 on the current token), state
-    [slots, K-1, C] updated in place.  Returns [T, C]."""
+    [slots, K-1, C] updated in place.  `longest`: new tokens of the longest sequence, where the caller knows it (else what it
+    can be); it chooses the kernel and changes no result.  Returns [T, C]."""
     if not x.is_cuda:
         return causal_conv1d_reference(x, w, state, q_start, seq_lens, slots, pre, post, silu)
     t, c = x.shape
@@ -82,7 +89,8 @@ def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, si
     rc = _lib.lib().zb_causal_conv1d(
         _ptr(x), x.stride(0), _ptr(pre), pre.stride(0) if pre is not None else 0, _ptr(post),
         post.stride(0) if post is not None else 0, _ptr(w), _ptr(out), out.stride(0), _ptr(state),
-        _ptr(q_start), _ptr(seq_lens), _ptr(slots), seq_lens.shape[0], t, c, k, 1 if silu else 0, _lib.stream_ptr())
+        _ptr(q_start), _ptr(seq_lens), _ptr(slots), seq_lens.shape[0], t, _longest(t, seq_lens, longest),
+        c, k, 1 if silu else 0, _lib.stream_ptr())
     _lib.check(rc, "zb_causal_conv1d")
     return out
 
