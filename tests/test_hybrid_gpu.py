@@ -1,5 +1,6 @@
 """Linear-attention / short-conv kernels and the hybrid models on a B200, against the float32
 PyTorch restatement of the same ops on the CPU."""
+import math
 import os
 
 import pytest
@@ -101,6 +102,40 @@ def test_gated_delta_chunks_match_the_walk(hk, hv, dk, dv, decay, monkeypatch):
     expect_close(res[0][0], res[1][0], atol=1e-2, rtol=1e-2, min_close=0.999)
     expect_close(res[0][1], res[1][1], atol=2e-5, rtol=1e-5, min_close=1.0)
     assert torch.equal(res[0][1][0], start[0])               # the empty sequence's slot
+
+
+def _scan_inputs(t, hk, hv, dk, dv):
+    o, val = 2 * hk * dk + hv * dv, hv * dv
+    proj = torch.randn(t, o + val + (2 * hv + 7) // 8 * 8, device=DEV).bfloat16()
+    return proj, (proj[:, :o], proj[:, o:o + val], proj[:, o + val:o + val + hv], proj[:, o + val + hv:o + val + 2 * hv], torch.randn(hv, device=DEV),
+                  torch.randn(hv, device=DEV), torch.ones(dv, device=DEV).bfloat16(), 1e-6)
+
+
+def test_rows_of_no_sequence_stay_as_they_are(monkeypatch):
+    """Token ranges that begin behind the first row and end in front of the last one: the rows around them are nobody's."""
+    torch.manual_seed(1)
+    monkeypatch.setattr(la, "_delta_in_chunks", lambda tokens, seqs: True)
+    hk, hv, dk, dv, first, lens = 1, 2, 64, 64, 70, [65, 3]
+    t = first + sum(lens) + 20
+    qs, sl, slots = (v.to(DEV) for v in _seq_meta(lens, [0, 9]))
+    _, args = _scan_inputs(t, hk, hv, dk, dv)
+    for front in (0, first):
+        rows = slice(front, front + sum(lens))
+        for name in ("scan", "conv"):
+            out = torch.full((t, hv * dv), 7.0, dtype=torch.bfloat16, device=DEV)
+            if name == "scan":
+                st = torch.ones(4, hv, dk, dv, device=DEV)
+                la.gated_delta_scan(*args, st, qs + front, sl, slots, hk, hv, dk, dv, out=out)
+                st2 = torch.ones(4, hv, dk, dv, device=DEV)
+                want = la.gated_delta_scan(*(a[rows] for a in args[:4]), *args[4:], st2, qs, sl, slots, hk, hv, dk, dv)
+            else:
+                x, w = args[0][:, :hv * dv], torch.randn(hv * dv, 4, device=DEV).bfloat16()
+                st = torch.ones(4, 3, hv * dv, dtype=torch.bfloat16, device=DEV)
+                la.causal_conv1d(x, w, st, qs + front, sl, slots, out=out)
+                st2 = torch.ones(4, 3, hv * dv, dtype=torch.bfloat16, device=DEV)
+                want = la.causal_conv1d(x[rows], w, st2, qs, sl, slots)
+            assert torch.equal(out[rows], want) and torch.equal(st, st2), name
+            assert bool((out[:rows.start] == 7).all() and (out[rows.stop:] == 7).all()), name
 
 
 @pytest.mark.parametrize("k,c", [(2, 8), (4, 1032), (5, 64)])

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(32 * kPrepWarps) zb_gdn_prep_kernel(const GdnC
     if (chunk_base(p.q_start, mid) <= cid) s = mid; else hi = mid;
   }
   const int t0 = p.q_start[s] + (cid - chunk_base(p.q_start, s)) * kC, n = min(kC, p.q_start[s + 1] - t0);
-  if (n <= 0) return;                                // the whole warp; no block barrier below
+  if (n <= 0 || t0 < p.q_start[s]) return;           // the whole warp; no block barrier below.  (In front of the first sequence: nobody's rows.)
 
   constexpr int kPieces = DK / 8;                    // 16-byte pieces of a row
 #pragma unroll
@@ -455,6 +455,7 @@ __global__ void __launch_bounds__(256) zb_gdn_norm_kernel(const GdnChunkParams p
   const long long first = (blockIdx.x * 256ll + threadIdx.x) / G, stride = gridDim.x * (256ll / G), items = static_cast<long long>(p.tokens) * p.hv;
   const long long t_step = stride / p.hv;
   const int h_step = static_cast<int>(stride - t_step * p.hv);
+  const int t_first = p.q_start[0], t_last = min(p.q_start[p.num_seqs], p.tokens);      // rows of no sequence stay as they are
   long long t = first / p.hv;
   int h = static_cast<int>(first - t * p.hv);
   const long long warp_first = (blockIdx.x * 256ll + (threadIdx.x & ~31)) / G;
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(256) zb_gdn_norm_kernel(const GdnChunkParams p
     bool in[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      in[k] = mine && t < p.tokens;
+      in[k] = mine && t >= t_first && t < t_last;
       y[k] = z[k] = make_uint4(0u, 0u, 0u, 0u);
       const long long col = static_cast<long long>(h) * p.dv + at;
       if (in[k]) {
