@@ -138,6 +138,32 @@ def test_rows_of_no_sequence_stay_as_they_are(monkeypatch):
             assert bool((out[:rows.start] == 7).all() and (out[rows.stop:] == 7).all()), name
 
 
+@pytest.mark.parametrize("what", ["q", "k", "v", "a", "b"])
+@pytest.mark.parametrize("junk", [float("nan"), float("inf"), -float("inf")])
+def test_gated_delta_chunks_are_causal_for_any_number(what, junk, monkeypatch):
+    """A token that is not finite changes no token in front of it, as in the walk token by token, wherever it lies in its chunk."""
+    torch.manual_seed(2)
+    hk, hv, dk, dv, t = 1, 2, 64, 64, 48
+    qs, sl, slots = (v.to(DEV) for v in _seq_meta([t], [0]))
+    proj, args = _scan_inputs(t, hk, hv, dk, dv)
+    o = 2 * hk * dk + hv * dv
+    col = {"q": 3, "k": hk * dk + 5, "v": 2 * hk * dk + 7, "a": o + hv * dv, "b": o + hv * dv + hv}[what]
+
+    def run(chunks):
+        monkeypatch.setattr(la, "_delta_in_chunks", lambda tokens, seqs: chunks)
+        return la.gated_delta_scan(*args, torch.zeros(4, hv, dk, dv, device=DEV), qs, sl, slots, hk, hv, dk, dv)
+    clean = run(True)
+    assert bool(clean.isfinite().all())
+    for at in (0, 5, 15, 16, 30, 47):
+        keep = proj[at, col].clone()
+        proj[at, col] = junk
+        got, walk = run(True), run(False)
+        assert torch.equal(got[:at], clean[:at]), at
+        if math.isnan(junk):
+            assert torch.equal(got.isnan(), walk.isnan()), at
+        proj[at, col] = keep
+
+
 @pytest.mark.parametrize("k,c", [(2, 8), (4, 1032), (5, 64)])
 def test_causal_conv1d_token_blocks(k, c):
     """Prompts cut along their tokens: block edges, sequences shorter than the taps, a continued and an empty one; the same roundings as
