@@ -559,7 +559,7 @@ int launch_scan(const GdnChunkParams& p, cudaStream_t s) {
   // A CTA asks for so much shared memory that an SM holds no more of them than its part: those that start while zb_gdn_prep still holds
   // most SMs would otherwise crowd on the others, where they share a tensor core for as long as they run: one sequence of 4096 tokens (64 CTAs)
   // 0.72 - 0.80 ms so, 0.48 on an SM each; eight of 512 (512 CTAs) 0.234 either way.
-  const long long ctas = static_cast<long long>(p.hv) * (p.dv / DVP) * p.num_seqs, per_sm = (ctas + 147) / 148;
+  const long long ctas = static_cast<long long>(p.hv) * (p.dv / DVP) * p.num_seqs, sms = std::max(1, zb_num_sms()), per_sm = (ctas + sms - 1) / sms;
   const int smem = std::max(kSmem, static_cast<int>(kShare / (per_sm + 1)) / 16 * 16 + 1024);
   zb_launch(zb_gdn_scan_kernel<DK, DVP>, dim3(p.hv * (p.dv / DVP), p.num_seqs), dim3(2 * DVP), smem, s, p);
   return static_cast<int>(cudaGetLastError());
@@ -577,7 +577,7 @@ int launch_chunked(const GdnChunkParams& p, cudaStream_t s) {
   const int lanes = p.dv <= 32 ? 4 : (p.dv <= 64 ? 8 : (p.dv <= 128 ? 16 : 32));
   const auto norm = lanes == 4 ? zb_gdn_norm_kernel<4> : (lanes == 8 ? zb_gdn_norm_kernel<8> : (lanes == 16 ? zb_gdn_norm_kernel<16> : zb_gdn_norm_kernel<32>));
   const long long blocks = (static_cast<long long>(p.tokens) * p.hv * lanes + 255) / 256;
-  zb_launch(norm, dim3(static_cast<unsigned>(std::min(148ll * 8, blocks))), dim3(256), 0, s, p);
+  zb_launch(norm, dim3(static_cast<unsigned>(std::min(zb_num_sms() * 8ll, blocks))), dim3(256), 0, s, p);
   zb_count_launch(3);
   return static_cast<int>(cudaGetLastError());
 }
