@@ -402,7 +402,8 @@ class Qwen35Model(LlamaModel):
                                silu=True, longest=meta.max_q_len)
         return la.gated_delta_scan(mix, proj[:, self.off_z:self.off_b], proj[:, self.off_a:self.off_a + self.hv_l],
                                    proj[:, self.off_b:self.off_a], w.a_log, w.dt_bias, w.norm_w, c.rms_norm_eps,
-                                   self.rec_state[i], q_start, seq_lens, slots, self.hk_l, self.hv_l, self.dk, self.dv)
+                                   self.rec_state[i], q_start, seq_lens, slots, self.hk_l, self.hv_l, self.dk, self.dv,
+                                   longest=meta.max_q_len)
 
     def layer(self, l: int, x, meta: AttnMeta, kv_cache):
         lw, c = self.layers[l], self.config

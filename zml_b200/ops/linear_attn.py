@@ -96,13 +96,15 @@ def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, si
 
 
 # ---------------------------------------------------------------------------- gated delta rule
-def _delta_in_chunks(tokens: int, seqs: int) -> bool:
-    """Whether a batch takes the chunked kernels (csrc/gated_delta_chunk.cu) instead of the walk token by token.  32 heads of 128, us
-    chunked / walked: 1 sequence of 8 / 16 / 64 tokens 27 / 17, 26 / 30, 27 / 107; 32 sequences of 2 / 4 / 8 / 100 tokens 49 / 28,
-    47 / 44, 48 / 78, 196 / 889; 4096 tokens 720 / 8179.  The walk takes 1.3 - 2 us a token, three launches 26 us; with many sequences
-    both are bound by the states they read and write."""
-    return tokens >= 16 * seqs or (seqs >= 16 and tokens >= 6 * seqs)
-
+def _delta_in_chunks(tokens: int, seqs: int, longest: Optional[int] = None) -> bool:
+    """Whether a batch takes the chunked kernels (csrc/gated_delta_chunk.cu) instead of the walk token by token.  The walk takes 1.3 - 1.6 us
+    a token of the longest sequence, the chunked kernels 19 us to begin with; with many sequences both are bound by the states they read and
+    write, 0.7 and 1.2 us a sequence.  32 heads of 128, us, chunked / walked: 1 sequence of 8 / 12 / 16 / 40 tokens 19 / 17, 19 / 23, 19 / 29,
+    23 / 67, of 4096 482 / 8179; 8 of 8 / 12 26 / 22, 28 / 30; 32 of 4 / 6 / 8 53 / 45, 53 / 61, 56 / 78; one of 200 beside 14 single tokens
+    57 / 329, one of 16 / 24 / 40 beside 31 51 / 45, 53 / 59, 55 / 87, one of 32 / 64 beside 127 174 / 151, 178 / 215."""
+    if longest is None:
+        longest = tokens // max(1, seqs)
+    return longest > 10 + 0.31 * seqs or (seqs >= 16 and tokens >= 6 * seqs)
 
 
 def _rows16(x) -> bool:
@@ -143,10 +145,10 @@ def gated_delta_scan_reference(mix, z, a, b, a_log, dt_bias, norm_w, eps, state,
 
 
 def gated_delta_scan(mix, z, a, b, a_log, dt_bias, norm_w, eps, state, q_start, seq_lens, slots,
-                     hk: int, hv: int, dk: int, dv: int, out=None):
+                     hk: int, hv: int, dk: int, dv: int, out=None, longest: Optional[int] = None):
     """mix [T, 2*hk*dk + hv*dv] = q | k | v after the conv; z [T, hv*dv]; a, b [T, hv] (same row
     stride); a_log, dt_bias float32 [hv]; norm_w [dv]; state float32 [slots, hv, dk, dv] updated
-    in place.  Returns the gated, normalised output [T, hv*dv]."""
+    in place.  `longest`: new tokens of the longest sequence, where the caller knows it (else an even batch is assumed).  Returns the gated, normalised output [T, hv*dv]."""
     if not mix.is_cuda:
         return gated_delta_scan_reference(mix, z, a, b, a_log, dt_bias, norm_w, eps, state, q_start, seq_lens,
                                           slots, hk, hv, dk, dv)
@@ -156,7 +158,7 @@ def gated_delta_scan(mix, z, a, b, a_log, dt_bias, norm_w, eps, state, q_start, 
     if out is None:
         out = torch.empty((t, hv * dv), dtype=torch.bfloat16, device=mix.device)
     n = seq_lens.shape[0]
-    if _delta_in_chunks(t, n) and _rows16(mix) and _rows16(z) and _rows16(out) and dk in (64, 128) and dv % 32 == 0 and dv <= 256:
+    if _delta_in_chunks(*((t, n) if longest is None else (t, n, longest))) and _rows16(mix) and _rows16(z) and _rows16(out) and dk in (64, 128) and dv % 32 == 0 and dv <= 256:
         l = _lib.lib()
         rec = torch.empty(l.zb_gated_delta_rec_bytes(t, n, hv), dtype=torch.uint8, device=mix.device)
         y = out if out.stride(0) == hv * dv else torch.empty((t, hv * dv), dtype=torch.bfloat16, device=mix.device)
