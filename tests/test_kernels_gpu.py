@@ -387,6 +387,23 @@ def test_paged_prefill_ignores_rows_behind_a_sequence(hd, junk):
         assert bool(clean.isfinite().all())
 
 
+@pytest.mark.parametrize("hd,hq,hkv", [(64, 8, 2), (64, 64, 8), (128, 4, 2), (256, 3, 1)])
+@pytest.mark.parametrize("seqs,longest", [(1, 1), (3, 128), (9, 129), (40, 64), (60, 100)])
+def test_paged_prefill_routes_of_short_prompts(hd, hq, hkv, seqs, longest):
+    """Short prompts, few and many, on whichever kernel the rule takes; `max_seq_len` and a wide block table change no more than the kernel."""
+    torch.manual_seed(seqs)
+    seq_lens = [longest - i * longest // (2 * seqs) for i in range(seqs)]
+    qs = [0]
+    for n in seq_lens:
+        qs.append(qs[-1] + n)
+    kc, vc, bt = _make_paged(seqs, seq_lens, hkv, hd, 64)
+    sl, qst, q = torch.tensor(seq_lens, dtype=torch.int32, device=DEV), torch.tensor(qs, dtype=torch.int32, device=DEV), _randn(qs[-1], hq, hd)
+    want = ref.paged_attention(q, kc, vc, bt, seq_lens, qs).float()
+    for kw in (dict(max_seq_len=longest), {}, dict(impl="mma")):
+        # probabilities and the result round to bf16: 2 * 2^-9 of a result of size one
+        expect_close(ops.paged_prefill(q, kc, vc, bt, sl, qst, **kw).float(), want, atol=2e-2, rtol=2e-2, min_close=ALL)
+
+
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("scale", [-0.2, 0.0])
 def test_paged_prefill_scale_below_zero(hd, scale):

@@ -101,7 +101,6 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                   const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   using S = Shape<HD>;
   constexpr int kStages = S::kStages, kHeads = S::kHeads;
-  zb_pdl_wait();                                     // q, the KV cache and the batch description come from preceding work
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* q_s = smem;                               // [kHeads][kQBytes]
@@ -125,36 +124,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int head0 = blockIdx.x * kHeads;
   const int kvh = head0 / group;
 
-  // The (sequence, 128-row query block) of this CTA.  Head pairs are the grid's fast index, and blocks are handed out from the end of
-  // the batch backwards, within a sequence from its last (longest) block: the short ones fill the last wave.
-  int seq = -1, qb = 0;
-  {
-    int rem = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
-    for (int i = 0; i < p.batch; ++i) {
-      const int nb = (p.q_start[i + 1] - p.q_start[i] + kRows - 1) / kRows;
-      if (rem < nb) {
-        seq = i;
-        qb = rem;
-        break;
-      }
-      rem -= nb;
-    }
-  }
-  if (seq < 0) return;                               // grid is an upper bound of the number of blocks
-  const int q_len = p.q_start[seq + 1] - p.q_start[seq];
-  const int len = p.seq_lens[seq];
-  const int ctx = len - q_len;
-  const int row_base = qb * kRows;
-  const int tok_base = p.q_start[seq] + row_base;
-  const int rows_valid = min(kRows, q_len - row_base);
-  const int last_key = min(len, ctx + row_base + kRows);                                    // exclusive
-  const int first_tile = p.window > 0 ? max(0, ctx + row_base - p.window + 1) / kKeys : 0;
-  const int n_tiles = (last_key + kKeys - 1) / kKeys - first_tile;
-  // Rows of the last page behind the sequence's end.  They hold whatever was there before, perhaps NaN, and a masked key's weight of zero
-  // does not make that zero: these rows of V are cleared in shared memory (those of K only reach scores that the mask replaces).
-  const int behind = (first_tile + n_tiles) * kKeys - len;
-
-  if (threadIdx.x == 0) {
+  if (warp == 4 * kHeads && lane == 0) {
     zb_mbar_init(q_full, 1);
     for (int s = 0; s < kStages; ++s) {
       zb_mbar_init(&k_full[s], 1);
@@ -171,9 +141,70 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
+    zb_fence_proxy_async_smem();                     // the first copies go out in front of the block's barrier
     zb_tma_prefetch_desc(&tmap_q);
     zb_tma_prefetch_desc(&tmap_k);
     zb_tma_prefetch_desc(&tmap_v);
+  }
+  zb_pdl_wait();                                     // q, the KV cache and the batch description come from preceding work
+
+  // The (sequence, 128-row query block) of this CTA.  Head pairs are the grid's fast index, and blocks are handed out from the end of
+  // the batch backwards, within a sequence from its last (longest) block: the short ones fill the last wave.  Every warp looks at 32
+  // sequences at a time, a lane each: one after the other, 40 sequences cost every CTA 3.4 us.
+  int seq = -1, qb = 0, q_first = 0, q_len = 0, len = 0;
+  {
+    int rem = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
+    for (int i0 = 0; i0 < p.batch; i0 += 32) {
+      const int i = i0 + lane, a = i < p.batch ? p.q_start[i] : 0, n = i < p.batch ? p.q_start[i + 1] - a : 0;
+      const int end = i < p.batch ? p.seq_lens[i] : 0, nb = max(0, n + kRows - 1) / kRows;
+      int upto = nb;                                 // blocks of the sequences up to this one
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, rem < upto);
+      if (hit != 0u) {
+        const int l = __ffs(hit) - 1;
+        seq = i0 + l;
+        qb = rem - __shfl_sync(0xffffffffu, upto - nb, l);
+        q_first = __shfl_sync(0xffffffffu, a, l);
+        q_len = __shfl_sync(0xffffffffu, n, l);
+        len = __shfl_sync(0xffffffffu, end, l);
+        break;
+      }
+      rem -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  if (seq < 0) return;                               // grid is an upper bound of the number of blocks
+  const int ctx = len - q_len;
+  const int row_base = qb * kRows;
+  const int tok_base = q_first + row_base;
+  const int rows_valid = min(kRows, q_len - row_base);
+  const int last_key = min(len, ctx + row_base + kRows);                                    // exclusive
+  const int first_tile = p.window > 0 ? max(0, ctx + row_base - p.window + 1) / kKeys : 0;
+  const int n_tiles = (last_key + kKeys - 1) / kKeys - first_tile;
+  // Rows of the last page behind the sequence's end.  They hold whatever was there before, perhaps NaN, and a masked key's weight of zero
+  // does not make that zero: these rows of V are cleared in shared memory (those of K only reach scores that the mask replaces).
+  const int behind = (first_tile + n_tiles) * kKeys - len;
+
+  const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
+  auto page_of = [&](int j) {
+    const int page = bt[first_tile + j];
+    return ZB_BC_OK(page, ZB_BC_PAGES, kKernelId, 10) ? page : 0;
+  };
+  auto load_page = [&](int page, uint32_t stage) {
+    zb_mbar_expect_tx(&k_full[stage], S::kKvBytes);
+    zb_tma_load_4d(k_s + stage * S::kKvBytes, &tmap_k, &k_full[stage], 0, page * kKeys, 0, kvh);
+    zb_mbar_expect_tx(&v_full[stage], S::kKvBytes);
+    zb_tma_load_4d(v_s + stage * S::kKvBytes, &tmap_v, &v_full[stage], 0, page * kKeys, 0, kvh);
+  };
+  if (warp == 4 * kHeads && lane == 0) {             // on their way while tensor memory is allocated
+    zb_mbar_expect_tx(q_full, kHeads * S::kQBytes);
+    for (int w = 0; w < kHeads; ++w)
+      for (int c = 0; c < S::kSubs; ++c)
+        zb_tma_load_2d(q_s + w * S::kQBytes + c * (kRows * 128), &tmap_q, q_full, (head0 + w) * HD + c * 64, tok_base);
+    if (n_tiles > 0) load_page(page_of(0), 0);
   }
   if (warp == 4 * kHeads + 1) {
     zb_tmem_alloc(tmem_holder, kTmemCols);
@@ -189,24 +220,17 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // ------------------------------------------------------------------ TMA producer
     bool ok = true;
     if (lane == 0) {
-      const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
-      zb_mbar_expect_tx(q_full, kHeads * S::kQBytes);
-      for (int w = 0; w < kHeads; ++w)
-        for (int c = 0; c < S::kSubs; ++c)
-          zb_tma_load_2d(q_s + w * S::kQBytes + c * (kRows * 128), &tmap_q, q_full, (head0 + w) * HD + c * 64, tok_base);
-      uint32_t stage = 0, phase = 0;
-      for (int j = 0; j < n_tiles; ++j) {
+      uint32_t stage = 1, phase = 0;
+      int next = n_tiles > 1 ? page_of(1) : 0;       // asked for a tile ahead: with two stages the wait below is what the loads hang on
+      for (int j = 1; j < n_tiles; ++j) {
+        const int page = next;
+        if (j + 1 < n_tiles) next = page_of(j + 1);
         if (j >= kStages && !zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag)) {
           *abort_where = 1u;
           ok = false;
           break;
         }
-        int page = bt[first_tile + j];
-        if (!ZB_BC_OK(page, ZB_BC_PAGES, kKernelId, 10)) page = 0;
-        zb_mbar_expect_tx(&k_full[stage], S::kKvBytes);
-        zb_tma_load_4d(k_s + stage * S::kKvBytes, &tmap_k, &k_full[stage], 0, page * kKeys, 0, kvh);
-        zb_mbar_expect_tx(&v_full[stage], S::kKvBytes);
-        zb_tma_load_4d(v_s + stage * S::kKvBytes, &tmap_v, &v_full[stage], 0, page * kKeys, 0, kvh);
+        load_page(page, stage);
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;

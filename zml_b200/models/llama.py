@@ -369,7 +369,7 @@ class LlamaModel(DecoderModel):
             from ..ops import baseline as impl
         if meta.is_prefill:
             a = impl.paged_prefill(q, kc, vc, meta.block_table, meta.seq_lens, meta.q_start,
-                                   window=c.sliding_window, total_q_blocks=meta.total_q_blocks)
+                                   window=c.sliding_window, total_q_blocks=meta.total_q_blocks, max_seq_len=meta.max_seq_len)
         else:
             a = impl.paged_decode(q, kc, vc, meta.block_table, meta.seq_lens, window=c.sliding_window,
                                   num_splits=meta.num_splits, max_seq_len=meta.max_seq_len)

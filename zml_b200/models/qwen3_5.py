@@ -386,7 +386,7 @@ class Qwen35Model(LlamaModel):
                              c.rms_norm_eps, True)
         if meta.is_prefill:
             a = ops.paged_prefill(q, kc, vc, meta.block_table, meta.seq_lens, meta.q_start,
-                                  total_q_blocks=meta.total_q_blocks)
+                                  total_q_blocks=meta.total_q_blocks, max_seq_len=meta.max_seq_len)
         else:
             a = ops.paged_decode(q, kc, vc, meta.block_table, meta.seq_lens, num_splits=meta.num_splits,
                                  max_seq_len=meta.max_seq_len)

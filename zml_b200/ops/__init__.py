@@ -401,17 +401,31 @@ def _tc_takes(q, k_cache, ext) -> bool:
     return ok and (ext is None or (q.shape[2] == 128 and bool(l.zb_paged_prefill_tc_ext_supported(ext.cap, ext.pair))))
 
 
+def _prefill_short(hq: int, hd: int, seqs: int, longest: int) -> bool:
+    """Whether the mma.sync kernel is the better one for prompts of at most two pages.  The tcgen05 kernel has one CTA per SM, of 128 rows of
+    two heads, with some 5 us before and behind its pages; the other one CTAs of 64 rows of one head, several on an SM.  us, mma.sync /
+    tcgen05, head_dim 64: one of 1 / 64 / 128 tokens with 32 heads 4.7 / 5.6, 5.4 / 6.2, 7.3 / 8.4 (129: 9.1 / 8.7); 4 of 128 with 16 / 32 heads
+    7.3 / 8.6, 8.9 / 8.7; 8 and 32 of 128 with 16 9.0 / 8.8, 19.9 / 18.3; 20 of 100 with 16 / 32 13.3 / 14.8, 21.0 / 23.1; 64 of 64 with 4 / 16 / 32
+    10.5 / 6.7, 17.9 / 21.1, 27.9 / 36.4.  head_dim 128: one of 1 / 128 with 32 5.7 / 6.9, 8.8 / 10.6, but 40 of 10 30.7 / 27.8.  head_dim
+    256: never."""
+    if hd == 256 or longest > 128:
+        return False
+    ctas, sms = seqs * hq // 2, _lib.lib().zb_num_sms()
+    return ctas <= 32 or (hd == 64 and (ctas > 2 * sms or (ctas > sms and (longest <= 64 or 2 * ctas <= 3 * sms))))
+
+
 def prefill_on_tc(q, k_cache, ext=None) -> bool:
     """Whether `paged_prefill` (impl "auto") runs the tcgen05 kernel."""
     return _ATTN_TC and _tc_takes(q, k_cache, ext)
 
 
 def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: float | None = None,
-                  window: int = 0, out=None, total_q_blocks: int | None = None, impl: str = "auto", ext=None):
+                  window: int = 0, out=None, total_q_blocks: int | None = None, impl: str = "auto", ext=None, max_seq_len: int | None = None):
     """Varlen causal attention of new tokens against the paged KV (which already holds them).
 
     q [T, hq, hd]; q_start int32 [B+1] (device); seq_lens int32 [B] = keys per sequence.
-    `impl`: "auto" (the tcgen05 kernel where it applies), "tc" (require it) or "mma" (the mma.sync kernel).  `ext` (CUDA
+    `max_seq_len`: keys of the longest sequence, where the caller knows it (else the block table's width); it chooses the kernel only.
+    `impl`: "auto" (the tcgen05 kernel where it applies and is the faster one), "tc" (require it) or "mma" (the mma.sync kernel).  `ext` (CUDA
     only, with `out`): a `gqa.AttnExt`, see `ops.gqa`.
     """
     if not _cuda(q):
@@ -436,7 +450,8 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
     tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or (out.data_ptr() % 16 == 0 and scale > 0))
     if impl == "tc" and not tc_ok:
         raise ValueError(f"the tensor-core prefill kernel does not take hq={hq} hkv={hkv} hd={hd} page={page}")
-    if tc_ok and (impl == "tc" or (impl == "auto" and _ATTN_TC)):
+    longest = max_seq_len if max_seq_len is not None else block_table.shape[1] * page
+    if tc_ok and (impl == "tc" or (impl == "auto" and _ATTN_TC and not (ext is None and _prefill_short(hq, hd, b, longest)))):
         rc = l.zb_paged_prefill_tc(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _ptr(seq_lens), _ptr(q_start), b, nqb, t,
             hq, hkv, hd, block_table.shape[1], q.stride(0), scale, int(window),

@@ -95,7 +95,7 @@ def paged_decode(q, k_cache, v_cache, block_table, seq_lens, scale=None, window=
 
 
 def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale=None, window=0, out=None,
-                  total_q_blocks=None):
+                  total_q_blocks=None, max_seq_len=None):
     t, hq, hd = q.shape
     page = k_cache.shape[1]
     res = torch.empty_like(q)

@@ -271,7 +271,7 @@ class Engine:
         meta = AttnMeta(True, dev[1], dev[2], bt_d, meta_d[nb + 1:2 * nb + 1], meta_d[:nb + 1],
                         total_q_blocks=sum((b - a + 63) // 64 for _, a, b in chunk),
                         logits_rows=meta_d[3 * nb + 1:] if rows else None, q_start_host=qs, seq_lens_host=sl,
-                        max_q_len=max(b - a for _, a, b in chunk),
+                        max_seq_len=max(sl), max_q_len=max(b - a for _, a, b in chunk),
                         state_slots=meta_d[2 * nb + 1:3 * nb + 1] if self.stateful else None)
         return dev[0], meta
 
