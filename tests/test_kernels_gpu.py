@@ -482,7 +482,7 @@ def test_rope_rows(hd, rot, hq, hkv, qk_norm):
     assert torch.equal(vc, vc2)
 
 
-@pytest.mark.parametrize("rows,vocab", [(1, 128256), (40, 32773), (200, 4099), (3, 1000), (2, 40)])
+@pytest.mark.parametrize("rows,vocab", [(1, 128256), (40, 32773), (200, 4099), (3, 1000), (2, 40), (5, 24001), (100, 65537)])
 def test_topk_and_argmax_over_clusters(rows, vocab):
     """Rows cut over clusters of 8, 4 and 1: random, rising, falling, all equal and lowest logits against a stable sort (equal logits: the
     lower index first)."""

@@ -392,42 +392,52 @@ __global__ void __launch_bounds__(128) zb_embedding_kernel(const int32_t* __rest
 // ---------------------------------------------------------------- argmax
 ZB_DEVICE void st_cluster(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
-// CTAs of a cluster that share a row of `vocab` logits: as many as keep the chip full without a second wave (1024 threads a CTA, two CTAs
-// an SM), at least 4096 logits each.  32 rows of 128256 by one CTA a row leave four fifths of the SMs idle.
-int row_cluster(int rows, int vocab) {
-  int c = 8;
-  while (c > 1 && (rows * c > 296 || vocab / c < 4096)) c >>= 1;
-  return c;
+// CTAs of a cluster that share a row of `vocab` logits: as many as keep the chip full without a second wave (at most `ctas`; 1024 threads a
+// CTA, two CTAs an SM), at least `least` logits each.  32 rows of 128256 by one CTA a row leave four fifths of the SMs idle.  As a power
+// of two.
+int row_cluster(int rows, int vocab, int ctas, int least) {
+  int log2 = 3;
+  while (log2 > 0 && ((static_cast<long long>(rows) << log2) > ctas || (vocab >> log2) < least)) --log2;
+  return log2;
 }
 
-// First index of the row maximum (ties -> lowest index, NaN ignored), f32 logits; a cluster per row, each CTA a slice of it.
-// One row of 128256: 3.5 us (one CTA: 14); 32 rows 5.1 (16).
+// First index of the row maximum (ties -> lowest index, NaN ignored), f32 logits.
 __global__ void __launch_bounds__(1024) zb_argmax_f32_kernel(const float* __restrict__ logits,
                                                              int32_t* __restrict__ out, int vocab,
-                                                             long long stride, int ctas) {
-  __shared__ float all_v[8];
-  __shared__ int all_i[8];
-  const int rank = blockIdx.x % ctas, row = blockIdx.x / ctas;
-  if (ctas > 1) zb_cluster_arrive();                 // every CTA runs before another one writes to its shared memory
+                                                             long long stride) {
   zb_pdl_launch();
   zb_pdl_wait();
-  const int per = (vocab + ctas - 1) / ctas, from = min(rank * per, vocab), n = min(per, vocab - from);
+  float best;
+  int bi;
+  zb_block_argmax_1024(logits + static_cast<size_t>(blockIdx.x) * stride, vocab, best, bi);
+  if (threadIdx.x == 0) out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
+}
+
+// The same with a cluster per row, each CTA a slice of it.  One row of 128256: 4.0 us (one CTA: 8.1); 32 rows 5.7 (8.4).
+__global__ void __launch_bounds__(1024) zb_argmax_cluster_kernel(const float* __restrict__ logits,
+                                                                 int32_t* __restrict__ out, int vocab,
+                                                                 long long stride, int log2_ctas) {
+  __shared__ float all_v[8];
+  __shared__ int all_i[8];
+  const int ctas = 1 << log2_ctas, rank = blockIdx.x & (ctas - 1), row = blockIdx.x >> log2_ctas;
+  zb_cluster_arrive();                               // every CTA runs before another one writes to its shared memory
+  zb_pdl_launch();
+  zb_pdl_wait();
+  const int per = (vocab + ctas - 1) >> log2_ctas, from = min(rank * per, vocab), n = min(per, vocab - from);
   float best;
   int bi;
   zb_block_argmax_1024(logits + static_cast<size_t>(row) * stride + from, n, best, bi);
   if (bi != 0x7fffffff) bi += from;
-  if (ctas > 1) {
-    zb_cluster_wait();
-    if (threadIdx.x == 0) {
-      st_cluster(zb_mapa(zb_smem_u32(&all_v[rank]), 0), __float_as_uint(best));
-      st_cluster(zb_mapa(zb_smem_u32(&all_i[rank]), 0), static_cast<uint32_t>(bi));
-    }
-    zb_cluster_arrive();
-    zb_cluster_wait();
-    if (rank == 0 && threadIdx.x == 0)
-      for (int c = 1; c < ctas; ++c) zb_argmax_merge(best, bi, all_v[c], all_i[c]);
+  zb_cluster_wait();
+  if (threadIdx.x == 0) {
+    st_cluster(zb_mapa(zb_smem_u32(&all_v[rank]), 0), __float_as_uint(best));
+    st_cluster(zb_mapa(zb_smem_u32(&all_i[rank]), 0), static_cast<uint32_t>(bi));
   }
-  if (rank == 0 && threadIdx.x == 0) out[row] = bi == 0x7fffffff ? 0 : bi;
+  zb_cluster_arrive();
+  zb_cluster_wait();
+  if (rank != 0 || threadIdx.x != 0) return;
+  for (int c = 1; c < ctas; ++c) zb_argmax_merge(best, bi, all_v[c], all_i[c]);
+  out[row] = bi == 0x7fffffff ? 0 : bi;
 }
 
 // ---------------------------------------------------------------- top-k + Gumbel-max
@@ -539,10 +549,10 @@ ZB_DEVICE void radix_topk(TopkShared& sh, const float* __restrict__ row, int len
 __global__ void __launch_bounds__(1024) zb_topk_sample_kernel(
     const float* __restrict__ logits, int32_t* __restrict__ out_token, float* __restrict__ topk_vals,
     int32_t* __restrict__ topk_idx, int rows, int vocab, long long stride, int k, float temperature,
-    uint64_t seed, uint64_t step, const unsigned long long* __restrict__ dev_rng, int ctas) {
+    uint64_t seed, uint64_t step, const unsigned long long* __restrict__ dev_rng, int log2_ctas) {
   __shared__ TopkShared sh;
   __shared__ int merge_n[8];
-  const int rank = blockIdx.x % ctas, row_i = blockIdx.x / ctas, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ctas = 1 << log2_ctas, rank = blockIdx.x & (ctas - 1), row_i = blockIdx.x >> log2_ctas, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (ctas > 1) zb_cluster_arrive();                 // every CTA runs before another one writes to its shared memory
   zb_pdl_launch();
   zb_pdl_wait();
@@ -553,7 +563,7 @@ __global__ void __launch_bounds__(1024) zb_topk_sample_kernel(
     step += dev_rng[1];
   }
   const float* row = logits + static_cast<size_t>(row_i) * stride;
-  const int per = ((vocab + ctas - 1) / ctas + 3) & ~3, from = min(rank * per, vocab), len = min(per, vocab - from);
+  const int per = (((vocab + ctas - 1) >> log2_ctas) + 3) & ~3, from = min(rank * per, vocab), len = min(per, vocab - from);
   const float* part = row + from;
   const bool vec = len >= 4096 && (reinterpret_cast<uintptr_t>(part) & 15) == 0;
   auto each = [&](auto&& f) {                        // f(index in the slice, logit), every element once
@@ -834,9 +844,12 @@ int zb_embedding(const int32_t* ids, const void* table, void* out, int tokens, i
 int zb_argmax_f32(const float* logits, int32_t* out, int rows, int vocab, long long stride,
                   void* stream) {
   if (rows <= 0) return 0;
-  const int ctas = row_cluster(rows, vocab);
-  zb_launch_cluster(zb_argmax_f32_kernel, dim3(rows * ctas), dim3(1024), 0, reinterpret_cast<cudaStream_t>(stream), ctas, logits, out, vocab, stride,
-                    ctas);
+  // A cluster's two barriers take 0.6 us, which short rows do not give back (1 CTA / cluster, us: a row of 16000 3.2 / 3.6, of 32000 3.8 / 3.4), nor
+  // rows of medium length that fill the SMs by themselves (64 of 32000: 4.1 / 4.6).
+  const int log2 = vocab < 32000 || (vocab < 65536 && 4 * static_cast<long long>(rows) > zb_num_sms()) ? 0 : row_cluster(rows, vocab, 2 * zb_num_sms(), 8000);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (log2 == 0) zb_launch(zb_argmax_f32_kernel, dim3(rows), dim3(1024), 0, s, logits, out, vocab, stride);
+  else zb_launch_cluster(zb_argmax_cluster_kernel, dim3(rows << log2), dim3(1024), 0, s, 1 << log2, logits, out, vocab, stride, log2);
   zb_count_launch(1);
   return static_cast<int>(cudaGetLastError());
 }
@@ -848,9 +861,9 @@ int zb_topk_sample_rng(const float* logits, int32_t* out_token, float* topk_vals
                        unsigned long long seed, unsigned long long step, const unsigned long long* dev_rng, void* stream) {
   if (rows <= 0) return 0;
   if (k < 1 || k > kMaxTopK) return -45;
-  const int ctas = row_cluster(rows, vocab);
-  zb_launch_cluster(zb_topk_sample_kernel, dim3(rows * ctas), dim3(1024), 0, reinterpret_cast<cudaStream_t>(stream), ctas, logits, out_token, topk_vals,
-                    topk_idx, rows, vocab, stride, k, temperature, static_cast<uint64_t>(seed), static_cast<uint64_t>(step), dev_rng, ctas);
+  const int log2 = row_cluster(rows, vocab, 2 * zb_num_sms(), 4096);
+  zb_launch_cluster(zb_topk_sample_kernel, dim3(rows << log2), dim3(1024), 0, reinterpret_cast<cudaStream_t>(stream), 1 << log2, logits, out_token, topk_vals,
+                    topk_idx, rows, vocab, stride, k, temperature, static_cast<uint64_t>(seed), static_cast<uint64_t>(step), dev_rng, log2);
   zb_count_launch(1);
   return static_cast<int>(cudaGetLastError());
 }
