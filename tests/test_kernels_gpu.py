@@ -462,7 +462,7 @@ def test_rope_kvwrite(layout, rot, qk_norm):
     assert torch.equal(vc, vc2)
 
 
-@pytest.mark.parametrize("hd,rot,hq,hkv,qk_norm", [(64, 64, 5, 1, True), (128, 128, 32, 8, False), (256, 64, 4, 1, True), (128, 48, 3, 3, True), (64, 16, 70, 2, False)])
+@pytest.mark.parametrize("hd,rot,hq,hkv,qk_norm", [(64, 64, 5, 1, True), (128, 128, 32, 8, False), (256, 64, 4, 1, True), (128, 48, 3, 3, True), (64, 16, 70, 2, False), (128, 128, 64, 8, True)])
 def test_rope_rows(hd, rot, hq, hkv, qk_norm):
     """The 16-byte form: heads that do not fill a warp, more pieces than threads, partial rotation, strided input, padding rows."""
     torch.manual_seed(hd + rot)

@@ -7,6 +7,8 @@
 // zml/attention/paged_attention.zig:218-254, swiglu
 // examples/llm/models/llama/model.zig:491-496, TokenEmbedding zml/nn.zig:432-436,
 // sampleTokens zml/nn.zig:1999-2033.
+#include <algorithm>
+
 #include "common.cuh"
 #include "host_api.h"
 
@@ -122,6 +124,7 @@ struct RopeParams {
   float norm_eps;
   int norm_unit_offset;
   long long num_slots;          // bounds for slot_mapping; slots < 0 are skipped (padding)
+  int share;                    // pieces of a token that one CTA takes (zb_rope_rows_kernel)
 };
 
 // One warp takes `heads_per_warp` consecutive heads (q, then k, then v) of one token: the rotation angles
@@ -277,9 +280,10 @@ __global__ void __launch_bounds__(512) zb_rope_rows_kernel(const RopeParams p) {
   // negative = padding row (no KV write); the checking build reports a slot past the cache instead of dropping it
   if (slot >= p.num_slots) (void)ZB_BC_OK(slot, p.num_slots, kKernelRopeKvWrite, 1);
   const bool slot_ok = slot >= 0 && slot < p.num_slots;
-  const int units = (p.hq + 2 * p.hkv) * kLanes;
-  const int rounded = (units + 31) & ~31;            // a warp goes through the loop as a whole
-  for (int u0 = threadIdx.x; u0 < rounded; u0 += blockDim.x) {
+  const int from = static_cast<int>(blockIdx.y) * p.share, units = min(from + p.share, (p.hq + 2 * p.hkv) * kLanes);
+  const int rounded = from + ((units - from + 31) & ~31);      // a warp goes through the loop as a whole
+  bool first = true;
+  for (int u0 = from + threadIdx.x; u0 < rounded; u0 += blockDim.x) {
     const bool in = u0 < units;
     const int u = in ? u0 : units - 1, h = u / kLanes, j = u - h * kLanes;
     const bool is_q = h < p.hq, is_k = !is_q && h < p.hq + p.hkv;
@@ -288,7 +292,8 @@ __global__ void __launch_bounds__(512) zb_rope_rows_kernel(const RopeParams p) {
     const int a0 = is_q || is_k ? v0 : 2 * j, a1 = is_q || is_k ? v1 : 2 * j + 1;
     const uint4* src = reinterpret_cast<const uint4*>(p.qkv + static_cast<size_t>(tok) * p.qkv_stride + static_cast<size_t>(h) * HD);
     uint4 x0 = src[a0], x1 = src[a1];
-    if (u0 == static_cast<int>(threadIdx.x)) {       // first turn: the angles, while the loads are on their way
+    if (first) {                                     // the angles, while the loads are on their way
+      first = false;
       for (int i = threadIdx.x; i < half; i += blockDim.x) {
         float s_, c_;
         sincosf(pos * p.inv_freq[i], &s_, &c_);
@@ -800,9 +805,13 @@ int zb_rope_kvwrite(const void* qkv, void* q_out, void* k_cache, void* v_cache,
   const auto at16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (layout == 0 && rot_dim % 16 == 0 && (hd == 64 || hd == 128 || hd == 256) && qkv_stride % 8 == 0 && at16(qkv) && at16(q_out) && at16(k_cache) &&
       at16(v_cache) && at16(q_norm_w) && at16(k_norm_w)) {
-    const int units = (hq + 2 * hkv) * (hd / 16), threads = units >= 512 ? 512 : (units + 31) / 32 * 32;
+    // Few tokens of more pieces than a CTA has threads: several CTAs a token, which a second turn of one makes wait (8 tokens of 64 + 8 + 8 heads
+    // of 128: 3.7 us in two turns).
+    const int units = (hq + 2 * hkv) * (hd / 16), parts = tokens <= 64 ? (units + 511) / 512 : 1;
+    p.share = ((units + parts - 1) / parts + 31) / 32 * 32;
+    const int threads = std::min(512, p.share);
     const auto kernel = hd == 64 ? zb_rope_rows_kernel<64> : (hd == 128 ? zb_rope_rows_kernel<128> : zb_rope_rows_kernel<256>);
-    zb_launch(kernel, dim3(tokens), dim3(threads), 0, reinterpret_cast<cudaStream_t>(stream), p);
+    zb_launch(kernel, dim3(tokens, parts), dim3(threads), 0, reinterpret_cast<cudaStream_t>(stream), p);
     zb_count_launch(1);
     return static_cast<int>(cudaGetLastError());
   }
