@@ -551,6 +551,18 @@ def test_moe_combine_adds_extra_and_residual():
     expect_close(cpu.float(), want.cpu(), atol=3e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 8, 9])
+def test_moe_combine_of_any_number_of_experts(k):
+    """Two, four or eight rows at a time: the sums are those of `finalize`, to the bit, half of the experts elsewhere."""
+    from zml_b200 import moe
+    torch.manual_seed(k)
+    t, d = 37, 1032
+    ids = torch.stack([torch.randperm(16, device=DEV)[:k] for _ in range(t)]).int()
+    _, _, pair_pos = moe.moe_align(ids, 4, 8)
+    o, w = _randn(t * k, d), torch.rand(t, k, device=DEV)
+    assert torch.equal(moe.combine(o, pair_pos, w, t, k), moe.finalize(o, pair_pos, w, t, k))
+
+
 @pytest.mark.parametrize("t,k,d", [(511, 8, 64), (512, 1, 2056), (515, 9, 1024), (700, 8, 4104)])
 def test_moe_gather_by_tokens(t, k, d):
     """The expert rows gathered from the tokens' side (from 512 tokens on) are those of the gather by rows, half of the experts elsewhere."""
