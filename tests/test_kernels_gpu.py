@@ -115,7 +115,8 @@ def test_gemm_emits_row_statistics_of_its_output(m, n, k):
 ALL = 1 - 1e-9      # every value: the share is a mean on the GPU, a product with 1 / n that may round below one
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (3, 17, 72), (8, 130, 1032), (5, 4800, 2056), (7, 96, 4096), (9, 17, 72), (12, 4800, 1032), (16, 130, 2056)])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 64), (3, 17, 72), (8, 130, 1032), (5, 4800, 2056), (7, 96, 4096), (9, 17, 72), (12, 4800, 1032), (16, 130, 2056),
+                                   (16, 4800, 2056), (13, 1040, 8200)])
 def test_gemm_few_tokens(m, n, k):
     """The kernel of up to 16 tokens at the edges of its tiles (16 rows, 1024 columns, more tiles than CTAs), all epilogues, against fp32:
     a bf16 rounding of a result of size one (2^-9), a few of them at size four."""

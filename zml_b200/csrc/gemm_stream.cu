@@ -1,4 +1,4 @@
-// out[M,N] = a[M,K] * w[N,K]^T for at most 8 tokens, 16 for smaller matrices: the decode step of a few sequences.
+// out[M,N] = a[M,K] * w[N,K]^T for at most 8 tokens, 12 or 16 for smaller matrices: the decode step of a few sequences.
 //
 // The work is to read the weights once.  The tcgen05 kernel (gemm_bf16.cu) streams them well once it runs, but each launch pays for
 // barriers, tensor memory, descriptors, a ring of tiles through shared memory and a cluster reduction, about 8 us that a matrix of 8 MB
@@ -26,7 +26,8 @@
 namespace {
 constexpr int kWarps = 8, kRowsTile = 16, kGroup = 4;                    // 32-column blocks of a warp's group
 constexpr int kMaxTokens = 16;
-constexpr long long kMaxLarge = 20ll << 20;                             // elements of a matrix for more than 8 tokens
+// elements of a matrix for 9 to 12 and for 13 to 16 tokens
+constexpr long long kMax12 = 64ll << 20, kMax16 = 40ll << 20;
 constexpr int kSpan = kWarps * kGroup * 32;                              // columns that the CTA's groups cover
 constexpr int kDepth = 3;
 constexpr int kRing = kDepth * 2 * kGroup * 32 * kWarps * 16;            // 96 KB
@@ -57,10 +58,20 @@ ZB_DEVICE void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
 
 // TT: tiles of 8 tokens
 template <int TT>
+struct __align__(16) StreamShared {
+  float part[2][kWarps][8 * TT][kRowsTile];          // rows of a token at `part_at`
+  float scale[8 * TT];
+};
+// Two CTAs share an SM (1 KB of its shared memory each is the system's).
+static_assert(2 * (kRing + sizeof(StreamShared<2>) + 1024) <= 228 * 1024, "two CTAs fit an SM");
+// Place of a weight row's sum among a token's 16: every other pair of tokens turned by 8, so that lanes of four tokens meet in pairs only.
+ZB_DEVICE int part_at(int token, int row) { return row ^ ((token & 2) << 2); }
+
+template <int TT>
 __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const StreamParams p) {
   extern __shared__ __align__(16) uint4 ring[];      // [kDepth][2 kGroup][threads]
-  __shared__ float part[2][kWarps][8 * TT][kRowsTile + 1];
-  __shared__ float scale[8 * TT];
+  __shared__ StreamShared<TT> sh;
+  auto& part = sh.part;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
   zb_pdl_launch();
   const int groups = (p.k + kSpan - 1) / kSpan;
@@ -113,7 +124,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
       if (t < p.m)
         for (int i = lane; i < p.in_parts; i += 32) ss += p.in_sumsq[static_cast<size_t>(i) * p.in_ld + t];
       ss = zb_warp_sum(ss);
-      if (lane == 0) scale[t] = rsqrtf(ss * p.in_inv_d + p.in_eps);
+      if (lane == 0) sh.scale[t] = rsqrtf(ss * p.in_inv_d + p.in_eps);
     }
   }
 
@@ -143,7 +154,8 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
     for (int t = 0; t < TT; ++t)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        part[buf][warp][8 * t + 2 * tq + (i & 1)][g + 8 * (i >> 1)] = acc[t][0][i] + acc[t][1][i];
+        const int token = 8 * t + 2 * tq + (i & 1);
+        part[buf][warp][token][part_at(token, g + 8 * (i >> 1))] = acc[t][0][i] + acc[t][1][i];
         acc[t][0][i] = acc[t][1][i] = 0.f;
       }
     __syncthreads();                                 // the other buffer is read by nobody any more once all warps are here
@@ -152,13 +164,14 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
       float v[2] = {0.f, 0.f};
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
-        v[0] += part[buf][w][tok][2 * pair];
-        v[1] += part[buf][w][tok][2 * pair + 1];
+        const float2 f = *reinterpret_cast<const float2*>(&part[buf][w][tok][part_at(tok, 2 * pair)]);
+        v[0] += f.x;
+        v[1] += f.y;
       }
       const bool in[2] = {row < p.n, row + 1 < p.n};
       if (p.in_sumsq != nullptr) {
-        v[0] *= scale[tok];
-        v[1] *= scale[tok];
+        v[0] *= sh.scale[tok];
+        v[1] *= sh.scale[tok];
       }
       if (p.act == ZB_ACT_SWIGLU) {
         if (in[1]) reinterpret_cast<__nv_bfloat16*>(p.out)[static_cast<size_t>(tok) * p.ldo + row / 2] = __float2bfloat16(zb_gate_act(v[0], ZB_ACT_SWIGLU) * v[1]);
@@ -196,11 +209,14 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
 }  // namespace
 
 // 1 when the kernel takes the problem.  9 to 16 tokens double the tokens' reads (as many bytes as the weights) and the MMAs, which a large
-// matrix does not hide.  12 / 16 tokens, us (tcgen05 kernel): 2048 x 2048 3.9 / 4.1 (7.5), 5120 x 2048 8.4 / 9.7 (9.9), 2048 x 8192
-// 9.8 / 10.5 (13.1), 4096 x 4096 10.4 / 11.3 (12.4); 6144 x 4096 15.0 / 16.7 (16.5), 16384 x 2048 16.8 / 19.7 (17.5), 28672 x 4096
-// 49.2 / 55.5 (44.2): the line lies between the last two groups.
+// matrix does not hide, nor a long row of which few CTAs have a share.  12 / 16 tokens, us (tcgen05 kernel): 2048 x 2048 3.7 / 3.7 (7.2),
+// 5120 x 2048 6.3 / 6.6 (10.2), 2048 x 8192 9.9 / 10.4 (13.4), 4096 x 4096 8.7 / 9.2 (12.9), 6144 x 4096 13.8 / 15.4 (18.1), 16384 x 2048
+// 14.9 / 16.3 (19.2); with statistics 4096 x 14336 30.1 / 33.3 (30.1), 12288 x 4096 27.9 / 30.7 (29.0), 28672 x 4096 54.8 / 58.5 (53.4);
+// 512 x 16384 13.2 / 14.9 (14.1).
 int zb_gemm_stream_wants(const void* a, const void* w, int m, int n, int k) {
-  return (m <= 8 || (m <= kMaxTokens && static_cast<long long>(n) * k <= kMaxLarge)) && n >= 16 && k >= 64 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+  const long long size = static_cast<long long>(n) * k;
+  const bool few = m <= 8 || (m <= 12 && size <= kMax12) || (m <= kMaxTokens && size <= kMax16 && (k <= 8192 || n >= 1024));
+  return few && n >= 16 && k >= 64 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 
 // The contract of the tcgen05 kernel's launch; epi->pf_* is ignored.  `out_parts`: parts written to epi->out_sumsq.
