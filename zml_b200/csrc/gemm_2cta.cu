@@ -394,8 +394,8 @@ zb_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
 }
 
-// Columns of the tiles.  A k-block takes 0.35 us with 256 columns and 0.31 with 64 (256 rows of A have to come either way), so narrow tiles
-// pay only where more SMs share the problem in the same single wave: 512 x 2048 x 2048 20.9 -> 15.3 us with the statistics, 512 x 3072 x
+// Columns of the tiles.  A k-block takes 0.35 us with 256 columns and 0.31 with 64 (measured; neither the bytes, 32 and 20 KB an SM, nor the
+// MMAs explain that the narrow one is no shorter: the cause is not known), so narrow tiles pay only where more SMs share the problem in the same single wave: 512 x 2048 x 2048 20.9 -> 15.3 us with the statistics, 512 x 3072 x
 // 2048 17.1 -> 15.3; but 1024 x 6144 x 4096 in three waves of 128 columns 62 us, in two of 256 46.
 int tile_columns(int m, int n, int num_sms) {
   const long long mt = (m + 2 * kBM - 1) / (2 * kBM);
@@ -421,9 +421,12 @@ int launch_tiles(const CUtensorMap& ta, const void* w, int ldw, Gemm2Params prm,
 }  // namespace
 
 // 1 when the two-SM kernel takes the problem: tokens as rows and at least one full tile of columns.  Above 128 tokens always (200 tokens, us,
-// here / one-SM kernel with weights as rows: 5120 x 2048 15 / 55, 28672 x 4096 60 / 139, 4096 x 14336 68 / 105).  From 65 on where the
-// estimates say so - a wave of tiles 0.32 us a k-block, the one-SM kernel 0.7 us for each k-block of 128 x 128 that an SM has to do and 7
-// more to begin with: 128 tokens, us: 5120 x 2048 15.1 / 17.1, 28672 x 4096 58 / 91, 2048 x 4096 22.6 / 16.0, 4096 x 14336 68 / 35.
+// here / one-SM kernel with weights as rows: 5120 x 2048 15 / 55, 28672 x 4096 60 / 139, 4096 x 14336 68 / 105) but where 257 to 384 tokens,
+// two tiles of 256 rows here and three of 128 there, meet so many columns that the padded rows are what counts (a vocabulary: 300 x
+// 128256 x 2048 183 / 175, with float32 outputs 221 / 194; 385 tokens 187 / 217).  From 65 on where the estimates say so - a wave of tiles
+// 0.32 us a k-block, the one-SM kernel 0.7 us for each k-block of 128 x 128 that an SM has to do and 6 more to begin with: 128 tokens, us:
+// 5120 x 2048 15.4 / 17.5, 6144 x 4096 25.8 / 29.0, 28672 x 4096 58 / 91, 3072 x 2048 with statistics 15.0 / 14.1, 2048 x 4096 22.6 / 16.0,
+// 4096 x 14336 68 / 37.
 // ZB_GEMM_2CTA=0 in the environment turns the kernel off.
 int zb_gemm_2cta_wants(int m, int n, int k, int num_sms) {
   static int enabled = -1;
@@ -432,10 +435,11 @@ int zb_gemm_2cta_wants(int m, int n, int k, int num_sms) {
     enabled = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
   if (!enabled || m <= 64 || n < 256 || k < 64) return 0;
+  if (m > 256 && m <= 384 && n >= 65536) return 0;
   if (m > 128) return 1;
   const int bn = tile_columns(m, n, num_sms), kb = (k + kBK - 1) / kBK;
   const int waves = ((n + bn - 1) / bn + num_sms / 2 - 1) / (num_sms / 2);
-  return 0.32 * waves * kb < 7. + 0.7 * ((n + 127) / 128) * kb / num_sms;
+  return 0.32 * waves * kb < 6. + 0.7 * ((n + 127) / 128) * kb / num_sms;
 }
 
 // out[M,N] = a[M,K] * w[N,K]^T (* row scale) (+ bias) (+ residual) or its SwiGLU: same contract as the one-SM
