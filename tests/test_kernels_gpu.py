@@ -388,6 +388,31 @@ def test_paged_prefill_ignores_rows_behind_a_sequence(hd, junk):
         assert bool(clean.isfinite().all())
 
 
+@pytest.mark.parametrize("cap", [0.0, 30.0])
+@pytest.mark.parametrize("window,keep", [(0, 0), (100, 3)])
+def test_paged_prefill_with_extensions_ignores_rows_behind_a_sequence(cap, window, keep):
+    """The same for the kernel with a score cap, a sink and kept first keys."""
+    from zml_b200.ops import gqa
+    torch.manual_seed(3)
+    parts = [(1, 0), (64, 64), (65, 63), (130, 70), (200, 120)]
+    q_lens, seq_lens = [n for n, _ in parts], [n + c for n, c in parts]
+    kc, vc, bt = _make_paged(len(parts), seq_lens, 2, 128, 64)
+    used = torch.zeros(kc.shape[:2], dtype=torch.bool, device=DEV)
+    for i, n in enumerate(seq_lens):
+        t = torch.arange(n, device=DEV)
+        used[bt[i, t // 64].long(), t % 64] = True
+    q, qs = _randn(sum(q_lens), 4, 128), [0]
+    for n in q_lens:
+        qs.append(qs[-1] + n)
+    sl, qst = torch.tensor(seq_lens, dtype=torch.int32, device=DEV), torch.tensor(qs, dtype=torch.int32, device=DEV)
+    ext, res = gqa.AttnExt(keep, cap, 1, 128, None, 0, 0), []
+    assert ops.prefill_on_tc(q, kc, ext)
+    for junk in (0.0, float("nan"), float("inf")):
+        kc[~used], vc[~used] = junk, -junk
+        res.append(ops.paged_prefill(q, kc, vc, bt, sl, qst, window=window, out=torch.empty_like(q), ext=ext))
+    assert bool(res[0].isfinite().all()) and torch.equal(res[1], res[0]) and torch.equal(res[2], res[0])
+
+
 @pytest.mark.parametrize("hd,hq,hkv", [(64, 8, 2), (64, 64, 8), (128, 4, 2), (256, 3, 1)])
 @pytest.mark.parametrize("seqs,longest", [(1, 1), (3, 128), (9, 129), (40, 64), (60, 100)])
 def test_paged_prefill_routes_of_short_prompts(hd, hq, hkv, seqs, longest):

@@ -195,7 +195,8 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   uint64_t* s_full = kv_empty + kStages;             // 2
   uint64_t* p_full = s_full + 2;                     // 2 (128 arrivals)
   uint64_t* o_ready = p_full + 2;                    // 2
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_ready + 2);
+  uint64_t* v_clean = o_ready + 2;                   // 1
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -232,6 +233,8 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   const int pooled = p.pool > 0 ? zb_pooled_visible(last_key - 1, p.window, p.pool) : 0;
   const ZbTileList tiles = zb_visible_tiles(first_key, p.keep, (last_key + kKeys - 1) / kKeys, kKeys, pooled);
   const int n_tiles = tiles.count;
+  // rows of the last page behind the sequence's end: cleared in V, since zero times what is there may be a NaN (see attention_prefill.cu)
+  const int behind = (last_key + kKeys - 1) / kKeys * kKeys - len;
 
   if (threadIdx.x == 0) {
     zb_mbar_init(q_full, 1);
@@ -245,6 +248,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       zb_mbar_init(&p_full[w], 128);
       zb_mbar_init(&o_ready[w], 1);
     }
+    zb_mbar_init(v_clean, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -296,6 +300,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         if (j >= kStages) {
           if (!zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag)) {
             *abort_where = 1u;
+            ok = false;
             break;
           }
         }
@@ -309,6 +314,20 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
           stage = 0;
           phase ^= 1u;
         }
+      }
+    }
+    if (n_tiles > 0 && behind > 0 && __all_sync(0xffffffffu, ok)) {
+      const int last = n_tiles - 1, at = last % kStages;
+      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / kStages) & 1u, abort_flag);
+      if (__all_sync(0xffffffffu, ok)) {
+        uint4* v = reinterpret_cast<uint4*>(v_s + at * kKvBytes) + (kKeys - behind) * 8;
+        for (int c = 0; c < kHD / 64; ++c)
+          for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+        zb_fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) zb_mbar_arrive(v_clean);
+      } else {
+        *abort_where = 8u;
       }
     }
   } else if (warp == 9) {
@@ -348,7 +367,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
           nstage = 0;
           nphase ^= 1u;
         }
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == n_tiles - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
           *abort_where = 4u;
           break;
         }
