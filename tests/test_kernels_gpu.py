@@ -338,13 +338,14 @@ def test_paged_prefill_tensor_core_kernel(hq, hkv, lens):
         expect_close(got.float(), old.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
 
 
-@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("hd,hq,hkv", [(64, 8, 2), (128, 8, 2), (256, 8, 2), (256, 3, 1)])
 @pytest.mark.parametrize("lens", [[(1, 0), (63, 0), (64, 1), (65, 63)], [(127, 0), (128, 64), (129, 191)], [(3, 4000), (260, 0)]])
-def test_paged_prefill_page_edges(hd, lens):
+def test_paged_prefill_page_edges(hd, hq, hkv, lens):
     """The tcgen05 prefill kernels at the edges of pages and query blocks, with scores that grow along the keys, so that a row's
-    reference moves again and again.  Probabilities are bf16 on both sides of P V: 2 * 2^-9 of a result of size one."""
+    reference moves again and again.  Probabilities and the result round to bf16, 2^-9 of each: at most 2^-8 of the largest value, which is
+    below 4.5; a wrong row is off by one and more."""
     torch.manual_seed(9)
-    hq, hkv, page = 8, 2, 64
+    page = 64
     q_lens, seq_lens = [a for a, _ in lens], [a + c for a, c in lens]
     kc, vc, bt = _make_paged(len(lens), seq_lens, hkv, hd, page)
     for i, n in enumerate(seq_lens):                # key t of a sequence is (1 + t / 40) times as large along one direction
@@ -360,7 +361,7 @@ def test_paged_prefill_page_edges(hd, lens):
     for window in (0, 1, 64, 100):
         got = ops.paged_prefill(q, kc, vc, bt, sl, qst, window=window, impl="tc")
         want = ref.paged_attention(q, kc, vc, bt, seq_lens, qs, window=window)
-        expect_close(got.float(), want.float(), atol=2e-2, rtol=2e-2, min_close=0.995)
+        expect_close(got.float(), want.float(), atol=2e-2, rtol=2e-2, min_close=ALL)
 
 
 @pytest.mark.parametrize("hd", [64, 128, 256])
@@ -490,7 +491,8 @@ def test_rope_kvwrite(layout, rot, qk_norm):
 
 @pytest.mark.parametrize("hd,rot,hq,hkv,qk_norm", [(64, 64, 5, 1, True), (128, 128, 32, 8, False), (256, 64, 4, 1, True), (128, 48, 3, 3, True), (64, 16, 70, 2, False), (128, 128, 64, 8, True)])
 def test_rope_rows(hd, rot, hq, hkv, qk_norm):
-    """The 16-byte form: heads that do not fill a warp, more pieces than threads, partial rotation, strided input, padding rows."""
+    """The 16-byte form: heads that do not fill a warp, more pieces than threads, partial rotation, strided input, padding rows.  Single values
+    differ by a rounding of the normalised value (2^-8 of up to twenty); a wrong 16-byte piece is off by one and more in all eight."""
     torch.manual_seed(hd + rot)
     t, page, pages = 9, 64, 3
     qkv = _randn(t, (hq + 2 * hkv) * hd + 16)[:, :(hq + 2 * hkv) * hd]
@@ -503,8 +505,9 @@ def test_rope_rows(hd, rot, hq, hkv, qk_norm):
     vc, kc2, vc2 = kc.clone(), kc.clone(), kc.clone()
     q = ops.rope_kvwrite(qkv, pos, slots, inv_freq, kc, vc, hq, hkv, hd, 0, rot, 1.1, qn, kn, 1e-6, qk_norm)
     q2 = ref.rope_kvwrite(qkv, pos, slots, inv_freq, kc2, vc2, hq, hkv, hd, 0, rot, 1.1, qn, kn, 1e-6, qk_norm)
-    expect_close(q.float(), q2.float(), atol=3e-2, rtol=2e-2, min_close=0.995)
-    expect_close(kc.float(), kc2.float(), atol=3e-2, rtol=2e-2, min_close=0.995)
+    for got, want in ((q, q2), (kc, kc2)):
+        expect_close(got.float(), want.float(), atol=3e-2, rtol=2e-2, min_close=0.995)
+        assert float((got.float() - want.float()).abs().reshape(-1, 8).mean(-1).max()) < 0.1
     assert torch.equal(vc, vc2)
 
 
