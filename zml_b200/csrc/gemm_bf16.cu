@@ -947,7 +947,6 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
         }
       };
       // bias / residual (read from this rank's memory) then store into `outp`
-      const bool rows16 = (prm.flags & 2) != 0;
       auto finish_chunk = [&](int c0, float (&v)[16]) {
         if constexpr (SWAP) {
           const float b = (prm.bias && p < prm.rows_p) ? __bfloat162float(prm.bias[p]) : 0.f;
@@ -965,7 +964,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           const size_t o = static_cast<size_t>(p) * prm.ldo + q;
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] *= row_scale;
-          if (rows16 && q + 16 <= prm.rows_q) {
+          if ((prm.flags & 2) != 0 && q + 16 <= prm.rows_q) {
             if (prm.bias) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) v[j] += __bfloat162float(prm.bias[q + j]);
@@ -1008,7 +1007,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           // p = output row m, q = output column n (16 consecutive columns per step)
           const int q = q0 + c0;
           const size_t o = static_cast<size_t>(p) * prm.ldo + q;
-          if (rows16 && q + 16 <= prm.rows_q) {
+          if ((prm.flags & 2) != 0 && q + 16 <= prm.rows_q) {
             if (prm.out_f32) {
               float4* op = reinterpret_cast<float4*>(reinterpret_cast<float*>(outp) + o);
 #pragma unroll
@@ -1049,7 +1048,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
           const int q = q0 + c0;
           if (p < prm.rows_p) {
             const size_t o = static_cast<size_t>(p) * prm.ldo + (q >> 1);
-            if (rows16 && q + 16 <= prm.rows_q) {
+            if ((prm.flags & 2) != 0 && q + 16 <= prm.rows_q) {
               uint32_t w[4];
 #pragma unroll
               for (int j = 0; j < 4; ++j)
@@ -1124,7 +1123,7 @@ zb_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p,
 #pragma unroll
             for (int e = 0; e < 4; ++e) bz[e] = (pb + e) < prm.rows_p ? __bfloat162float(prm.bias[pb + e]) : 0.f;
           }
-          const bool vec = (pb + 3) < prm.rows_p && rows16;
+          const bool vec = (pb + 3) < prm.rows_p && (prm.ldo % 4) == 0;
           // residual loads first, all of them: `out` may alias `residual`, which would otherwise
           // order every load behind the previous column's store
           uint2 rres[kCols];
@@ -1803,6 +1802,12 @@ int gemm_impl(const void* a, const void* w, void* out, const void* residual, con
     grid = num_sms;
     upc = rr * ((k + kBlockK - 1) / kBlockK);
   }
+  const bool rows16 = zb_gemm_rows16(out, residual, ldo, out_f32);
+  if (sw && bn <= 64 && cluster == 1 && !rows16) {      // whole tiles: the fix-up of split ones moves several columns at a time
+    rr = (tiles + num_sms - 1) / num_sms;
+    grid = tiles < num_sms ? tiles : num_sms;
+    upc = rr * ((k + kBlockK - 1) / kBlockK);
+  }
   if (cluster == 1 && rr == 0 && static_cast<size_t>(grid) * 2 * bn * kBlockP * sizeof(float) > scratch_bytes) return -13;
   if (tiles > counters_len) return -14;
   GemmParams prm;
@@ -1820,7 +1825,7 @@ int gemm_impl(const void* a, const void* w, void* out, const void* residual, con
   prm.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   prm.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   prm.out_f32 = out_f32;
-  prm.flags = static_w | (zb_gemm_rows16(out, residual, ldo, out_f32) ? 2 : 0);
+  prm.flags = static_w | (rows16 ? 2 : 0);
   prm.l2_prefetch = l2_prefetch_tiles(sw, bn, grid, rr);
   prm.timeline = next_timeline(grid);
   prm.group_p = (band != nullptr && band->mode != 0) ? 8 : 16;     // band pipeline: bands finish (and start) in groups of 8
