@@ -59,13 +59,15 @@ ZB_DEVICE void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, ui
 // TT: tiles of 8 tokens
 template <int TT>
 struct __align__(16) StreamShared {
-  float part[2][kWarps][8 * TT][kRowsTile];          // rows of a token at `part_at`
+  float part[2][kWarps][8 * TT][kRowsTile + (TT == 1 ? 1 : 0)];      // rows of a token at `part_at`
   float scale[8 * TT];
 };
 // Two CTAs share an SM (1 KB of its shared memory each is the system's).
 static_assert(2 * (kRing + sizeof(StreamShared<2>) + 1024) <= 228 * 1024, "two CTAs fit an SM");
-// Place of a weight row's sum among a token's 16: every other pair of tokens turned by 8, so that lanes of four tokens meet in pairs only.
-ZB_DEVICE int part_at(int token, int row) { return row ^ ((token & 2) << 2); }
+// Place of a weight row's sum among a token's 16.  Against bank conflicts one tile of tokens has a column of padding; two tiles have no room
+// for it, there every other pair of tokens is turned by 8.
+template <int TT>
+ZB_DEVICE int part_at(int token, int row) { return TT == 1 ? row : row ^ ((token & 2) << 2); }
 
 template <int TT>
 __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const StreamParams p) {
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int token = 8 * t + 2 * tq + (i & 1);
-        part[buf][warp][token][part_at(token, g + 8 * (i >> 1))] = acc[t][0][i] + acc[t][1][i];
+        part[buf][warp][token][part_at<TT>(token, g + 8 * (i >> 1))] = acc[t][0][i] + acc[t][1][i];
         acc[t][0][i] = acc[t][1][i] = 0.f;
       }
     __syncthreads();                                 // the other buffer is read by nobody any more once all warps are here
@@ -164,9 +166,8 @@ __global__ void __launch_bounds__(32 * kWarps, 2) zb_gemm_stream_kernel(const St
       float v[2] = {0.f, 0.f};
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
-        const float2 f = *reinterpret_cast<const float2*>(&part[buf][w][tok][part_at(tok, 2 * pair)]);
-        v[0] += f.x;
-        v[1] += f.y;
+        v[0] += part[buf][w][tok][part_at<TT>(tok, 2 * pair)];
+        v[1] += part[buf][w][tok][part_at<TT>(tok, 2 * pair + 1)];
       }
       const bool in[2] = {row < p.n, row + 1 < p.n};
       if (p.in_sumsq != nullptr) {
