@@ -321,6 +321,33 @@ def test_latent_decode_chunks_and_padding_rows(target):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name", ["tiles", "all", "bigrot"])
+def test_the_next_sequence_of_a_batch_does_not_show(name):
+    """Keys and values of a sequence that are not finite change no other one's result, wherever that one ends in a tile."""
+    d, counts = DIMS[name], (70, 1, 64, 130, 40)
+    torch.manual_seed(1)
+    dim_p, rot_p = -(-d.dim // 64) * 64, -(-d.rot // 64) * 64
+    qs, sl = varlen(counts, (0,) * len(counts), "cuda")
+    t, starts = sum(counts), qs.tolist()
+    qp = torch.zeros((t, d.heads, dim_p + rot_p), device="cuda", dtype=BF16)
+    qp[..., :d.dim].normal_()
+    qp[..., dim_p:dim_p + d.rot].normal_()
+    lat_rows = torch.zeros((t, 64 + rot_p), device="cuda", dtype=BF16)
+    lat_rows[:, 64:64 + d.rot].normal_()
+    kv = torch.randn((t, d.heads * (d.dim + d.vdim)), device="cuda").to(BF16)
+    meta = SimpleNamespace(q_start=qs, seq_lens=sl, q_start_host=starts, plans={})
+    plan = qs, i32([0] * len(counts), "cuda"), t
+    clean = lat.attend_expanded(qp, None, lat_rows, kv, 64, plan, meta, d)
+    assert torch.isfinite(clean.float()).all()
+    for bad in range(1, len(counts)):
+        rows = slice(starts[bad], starts[bad + 1])
+        spoilt = kv.clone()
+        spoilt[rows] = float("nan")
+        got = lat.attend_expanded(qp, None, lat_rows, spoilt, 64, plan, meta, d)
+        assert torch.equal(got[:rows.start], clean[:rows.start]) and torch.equal(got[rows.stop:], clean[rows.stop:]), bad
+
+
+@pytest.mark.gpu
 def test_prefill_kernel_and_latent_space_agree_on_a_batch():
     """Several blocks of 256 queries, sequences that start inside a window, rows at every block's edge."""
     d = dims(6, 128, 64, 128, 256, 96, 300, 0.06)

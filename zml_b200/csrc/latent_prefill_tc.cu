@@ -71,7 +71,8 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
   uint64_t* s_full = kv_empty + STAGES;              // 2
   uint64_t* p_full = s_full + 2;                     // 2 (128 arrivals)
   uint64_t* o_ready = p_full + 2;                    // 2
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_ready + 2);
+  uint64_t* v_clean = o_ready + 2;                   // 1
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -97,6 +98,8 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
     t_end[w] = (min(len, base + kQRows) + kKeys - 1) / kKeys;
   }
   const int tile0 = t_begin[0], tile1 = t_end[n_pipe - 1];
+  // Rows of the last tile behind the sequence's end are the next sequence's: cleared in V, since a weight of zero does not make a NaN zero.
+  const int behind = tile1 * kKeys - len;
 
   if (threadIdx.x == 0) {
     zb_mbar_init(q_full, 1);
@@ -110,6 +113,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       zb_mbar_init(&p_full[w], 128);
       zb_mbar_init(&o_ready[w], 1);
     }
+    zb_mbar_init(v_clean, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -129,6 +133,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
+    bool ok = true;
     if (lane == 0) {
       zb_mbar_expect_tx(q_full, n_pipe * kQBytes);
       for (int w = 0; w < n_pipe; ++w)
@@ -139,6 +144,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
         if (j - tile0 >= STAGES) {
           if (!zb_mbar_wait(&kv_empty[stage], phase ^ 1u, abort_flag)) {
             *abort_where = 1u;
+            ok = false;
             break;
           }
         }
@@ -156,6 +162,20 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           stage = 0;
           phase ^= 1u;
         }
+      }
+    }
+    if (tile0 < tile1 && behind > 0 && __all_sync(0xffffffffu, ok)) {
+      const int last = tile1 - 1 - tile0, at = last % STAGES;
+      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / STAGES) & 1u, abort_flag);
+      if (__all_sync(0xffffffffu, ok)) {
+        uint4* v = reinterpret_cast<uint4*>(v_s + at * kVBytes) + (kKeys - behind) * 8;      // the swizzle stays within a row of 128 bytes
+        for (int c = 0; c < NV; ++c)
+          for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+        zb_fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) zb_mbar_arrive(v_clean);
+      } else {
+        *abort_where = 8u;
       }
     }
   } else if (warp == 9) {
@@ -193,7 +213,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           nstage = 0;
           nphase ^= 1u;
         }
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == tile1 - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
           *abort_where = 4u;
           break;
         }
