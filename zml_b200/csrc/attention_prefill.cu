@@ -114,8 +114,8 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* s_full = kv_empty + kStages;             // [2 heads][2 buffers]
   uint64_t* p_full = s_full + 4;                     // [2 heads][2 buffers], four warps
   uint64_t* o_ready = p_full + 4;                    // 2
-  uint64_t* v_clean = o_ready + 2;                   // 1
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
+  uint64_t* v_raw = o_ready + 2;                     // 1: V of a page that is cleared behind the sequence's end
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_raw + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -137,7 +137,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     zb_mbar_init(&o_ready[0], 1);
     zb_mbar_init(&o_ready[1], 1);
-    zb_mbar_init(v_clean, 1);
+    zb_mbar_init(v_raw, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -151,12 +151,11 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   // The (sequence, 128-row query block) of this CTA.  Head pairs are the grid's fast index, and blocks are handed out from the end of
   // the batch backwards, within a sequence from its last (longest) block: the short ones fill the last wave.  Every warp looks at 32
   // sequences at a time, a lane each: one after the other, 40 sequences cost every CTA 3.4 us.
-  int seq = -1, qb = 0, q_first = 0, q_len = 0, len = 0;
+  int seq = -1, qb = 0;
   {
     int rem = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
     for (int i0 = 0; i0 < p.batch; i0 += 32) {
-      const int i = i0 + lane, a = i < p.batch ? p.q_start[i] : 0, n = i < p.batch ? p.q_start[i + 1] - a : 0;
-      const int end = i < p.batch ? p.seq_lens[i] : 0, nb = max(0, n + kRows - 1) / kRows;
+      const int i = i0 + lane, nb = i < p.batch ? max(0, p.q_start[i + 1] - p.q_start[i] + kRows - 1) / kRows : 0;
       int upto = nb;                                 // blocks of the sequences up to this one
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -166,17 +165,15 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint32_t hit = __ballot_sync(0xffffffffu, rem < upto);
       if (hit != 0u) {
         const int l = __ffs(hit) - 1;
-        seq = i0 + l;
-        qb = rem - __shfl_sync(0xffffffffu, upto - nb, l);
-        q_first = __shfl_sync(0xffffffffu, a, l);
-        q_len = __shfl_sync(0xffffffffu, n, l);
-        len = __shfl_sync(0xffffffffu, end, l);
+        seq = i0 + l;                                // what the loops go by is found alike in all lanes (a value out of a shuffle cost them 0.7 %)
+        qb = rem - __reduce_add_sync(0xffffffffu, lane < l ? nb : 0);
         break;
       }
-      rem -= __shfl_sync(0xffffffffu, upto, 31);
+      rem -= __reduce_add_sync(0xffffffffu, nb);
     }
   }
   if (seq < 0) return;                               // grid is an upper bound of the number of blocks
+  const int q_first = p.q_start[seq], q_len = p.q_start[seq + 1] - q_first, len = p.seq_lens[seq];
   const int ctx = len - q_len;
   const int row_base = qb * kRows;
   const int tok_base = q_first + row_base;
@@ -185,7 +182,9 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int first_tile = p.window > 0 ? max(0, ctx + row_base - p.window + 1) / kKeys : 0;
   const int n_tiles = (last_key + kKeys - 1) / kKeys - first_tile;
   // Rows of the last page behind the sequence's end.  They hold whatever was there before, perhaps NaN, and a masked key's weight of zero
-  // does not make that zero: these rows of V are cleared in shared memory (those of K only reach scores that the mask replaces).
+  // does not make that zero: these rows of V are cleared in shared memory (those of K only reach scores that the mask replaces).  The page
+  // comes with a barrier of its own, and the producer warp arrives on the ring's behind its stores: the MMA threads know nothing of it (a
+  // condition in their loop cost 0.4 %).
   const int behind = (first_tile + n_tiles) * kKeys - len;
 
   const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
@@ -193,18 +192,19 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const int page = bt[first_tile + j];
     return ZB_BC_OK(page, ZB_BC_PAGES, kKernelId, 10) ? page : 0;
   };
-  auto load_page = [&](int page, uint32_t stage) {
+  auto load_page = [&](int page, uint32_t stage, bool last) {
+    uint64_t* v_bar = last && behind > 0 ? v_raw : &v_full[stage];
     zb_mbar_expect_tx(&k_full[stage], S::kKvBytes);
     zb_tma_load_4d(k_s + stage * S::kKvBytes, &tmap_k, &k_full[stage], 0, page * kKeys, 0, kvh);
-    zb_mbar_expect_tx(&v_full[stage], S::kKvBytes);
-    zb_tma_load_4d(v_s + stage * S::kKvBytes, &tmap_v, &v_full[stage], 0, page * kKeys, 0, kvh);
+    zb_mbar_expect_tx(v_bar, S::kKvBytes);
+    zb_tma_load_4d(v_s + stage * S::kKvBytes, &tmap_v, v_bar, 0, page * kKeys, 0, kvh);
   };
   if (warp == 4 * kHeads && lane == 0) {             // on their way while tensor memory is allocated
     zb_mbar_expect_tx(q_full, kHeads * S::kQBytes);
     for (int w = 0; w < kHeads; ++w)
       for (int c = 0; c < S::kSubs; ++c)
         zb_tma_load_2d(q_s + w * S::kQBytes + c * (kRows * 128), &tmap_q, q_full, (head0 + w) * HD + c * 64, tok_base);
-    if (n_tiles > 0) load_page(page_of(0), 0);
+    if (n_tiles > 0) load_page(page_of(0), 0, n_tiles == 1);
   }
   if (warp == 4 * kHeads + 1) {
     zb_tmem_alloc(tmem_holder, kTmemCols);
@@ -230,7 +230,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           ok = false;
           break;
         }
-        load_page(page, stage);
+        load_page(page, stage, j == n_tiles - 1);
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
@@ -238,15 +238,15 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
     }
     if (n_tiles > 0 && behind > 0 && __all_sync(0xffffffffu, ok)) {
-      const int last = n_tiles - 1, at = last % kStages;
-      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / kStages) & 1u, abort_flag);
+      const int at = (n_tiles - 1) % kStages;
+      ok = zb_mbar_wait(v_raw, 0u, abort_flag);
       if (__all_sync(0xffffffffu, ok)) {
         uint4* v = reinterpret_cast<uint4*>(v_s + at * S::kKvBytes) + (kKeys - behind) * 8;      // the swizzle stays within a row of 128 bytes
         for (int c = 0; c < S::kSubs; ++c)
           for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
         zb_fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) zb_mbar_arrive(v_clean);
+        if (lane == 0) zb_mbar_arrive(&v_full[at]);
       } else {
         *abort_where = 7u;
       }
@@ -284,7 +284,7 @@ zb_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         where = 3u;
       }
       for (int j = 0; where == 0u && j < n_tiles; ++j) {
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == n_tiles - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
           where = 4u;
           break;
         }

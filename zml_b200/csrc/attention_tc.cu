@@ -195,8 +195,8 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   uint64_t* s_full = kv_empty + kStages;             // 2
   uint64_t* p_full = s_full + 2;                     // 2 (128 arrivals)
   uint64_t* o_ready = p_full + 2;                    // 2
-  uint64_t* v_clean = o_ready + 2;                   // 1
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
+  uint64_t* v_raw = o_ready + 2;                     // 1: V of a page that is cleared behind the sequence's end
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_raw + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -248,7 +248,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       zb_mbar_init(&p_full[w], 128);
       zb_mbar_init(&o_ready[w], 1);
     }
-    zb_mbar_init(v_clean, 1);
+    zb_mbar_init(v_raw, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -308,8 +308,9 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         if (!ZB_BC_OK(page, ZB_BC_PAGES, kKernelId, 10)) page = 0;
         zb_mbar_expect_tx(&k_full[stage], kKvBytes);
         zb_tma_load_4d(k_s + stage * kKvBytes, &tmap_k, &k_full[stage], 0, page * kKeys, 0, kvh);
-        zb_mbar_expect_tx(&v_full[stage], kKvBytes);
-        zb_tma_load_4d(v_s + stage * kKvBytes, &tmap_v, &v_full[stage], 0, page * kKeys, 0, kvh);
+        uint64_t* v_bar = j == n_tiles - 1 && behind > 0 ? v_raw : &v_full[stage];
+        zb_mbar_expect_tx(v_bar, kKvBytes);
+        zb_tma_load_4d(v_s + stage * kKvBytes, &tmap_v, v_bar, 0, page * kKeys, 0, kvh);
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
@@ -317,15 +318,15 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       }
     }
     if (n_tiles > 0 && behind > 0 && __all_sync(0xffffffffu, ok)) {
-      const int last = n_tiles - 1, at = last % kStages;
-      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / kStages) & 1u, abort_flag);
+      const int at = (n_tiles - 1) % kStages;
+      ok = zb_mbar_wait(v_raw, 0u, abort_flag);
       if (__all_sync(0xffffffffu, ok)) {
         uint4* v = reinterpret_cast<uint4*>(v_s + at * kKvBytes) + (kKeys - behind) * 8;
         for (int c = 0; c < kHD / 64; ++c)
           for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
         zb_fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) zb_mbar_arrive(v_clean);
+        if (lane == 0) zb_mbar_arrive(&v_full[at]);
       } else {
         *abort_where = 8u;
       }
@@ -367,7 +368,7 @@ zb_paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
           nstage = 0;
           nphase ^= 1u;
         }
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == n_tiles - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
           *abort_where = 4u;
           break;
         }
@@ -652,7 +653,7 @@ int zb_paged_prefill_tc(const void* q, const void* k_cache, const void* v_cache,
   if (!zb_paged_prefill_tc_supported(num_q_heads, num_kv_heads, head_dim, kKeys) || (ext != nullptr && head_dim != kHD)) return -32;
   ZbDeviceState* st = zb_device_state();
   if (!st) return -20;
-  if (ext == nullptr && (reinterpret_cast<uintptr_t>(out) & 15) != 0) return -33;
+  if (ext == nullptr && ((reinterpret_cast<uintptr_t>(out) & 15) != 0 || !(scale > 0.f))) return -33;
   total_q_blocks128 = std::min(total_q_blocks128, total_tokens / kQRows + batch);      // a caller may count blocks of 64 rows
   if (ext == nullptr)
     return zb_prefill_plain(q, k_cache, v_cache, out, block_table, seq_lens, q_start, batch, total_q_blocks128, total_tokens, num_q_heads,

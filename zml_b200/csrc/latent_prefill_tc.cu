@@ -71,8 +71,8 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
   uint64_t* s_full = kv_empty + STAGES;              // 2
   uint64_t* p_full = s_full + 2;                     // 2 (128 arrivals)
   uint64_t* o_ready = p_full + 2;                    // 2
-  uint64_t* v_clean = o_ready + 2;                   // 1
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_clean + 1);
+  uint64_t* v_raw = o_ready + 2;                     // 1: V of a tile that is cleared behind the sequence's end
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_raw + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
   volatile uint32_t* abort_where = tmem_holder + 2;
 
@@ -113,7 +113,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       zb_mbar_init(&p_full[w], 128);
       zb_mbar_init(&o_ready[w], 1);
     }
-    zb_mbar_init(v_clean, 1);
+    zb_mbar_init(v_raw, 1);
     *abort_flag = 0u;
     *abort_where = 0u;
     zb_mbar_fence_init();
@@ -155,9 +155,10 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           if (c < p.nn) zb_tma_load_2d(dst, &tmap_kv, &k_full[stage], head * p.dim + c * 64, row);
           else zb_tma_load_2d(dst, &tmap_shared, &k_full[stage], p.rot_out + (c - p.nn) * 64, row);
         }
-        zb_mbar_expect_tx(&v_full[stage], kVBytes);
+        uint64_t* v_bar = j == tile1 - 1 && behind > 0 ? v_raw : &v_full[stage];
+        zb_mbar_expect_tx(v_bar, kVBytes);
         for (int c = 0; c < NV; ++c)
-          zb_tma_load_2d(v_s + stage * kVBytes + c * kKvSub, &tmap_kv, &v_full[stage], p.heads * p.dim + head * p.vdim + c * 64, row);
+          zb_tma_load_2d(v_s + stage * kVBytes + c * kKvSub, &tmap_kv, v_bar, p.heads * p.dim + head * p.vdim + c * 64, row);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1u;
@@ -165,15 +166,15 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
       }
     }
     if (tile0 < tile1 && behind > 0 && __all_sync(0xffffffffu, ok)) {
-      const int last = tile1 - 1 - tile0, at = last % STAGES;
-      ok = zb_mbar_wait(&v_full[at], static_cast<uint32_t>(last / STAGES) & 1u, abort_flag);
+      const int at = (tile1 - 1 - tile0) % STAGES;
+      ok = zb_mbar_wait(v_raw, 0u, abort_flag);
       if (__all_sync(0xffffffffu, ok)) {
         uint4* v = reinterpret_cast<uint4*>(v_s + at * kVBytes) + (kKeys - behind) * 8;      // the swizzle stays within a row of 128 bytes
         for (int c = 0; c < NV; ++c)
           for (int i = lane; i < behind * 8; i += 32) v[c * kKeys * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
         zb_fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) zb_mbar_arrive(v_clean);
+        if (lane == 0) zb_mbar_arrive(&v_full[at]);
       } else {
         *abort_where = 8u;
       }
@@ -213,7 +214,7 @@ zb_latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __
           nstage = 0;
           nphase ^= 1u;
         }
-        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag) || (behind > 0 && j == tile1 - 1 && !zb_mbar_wait(v_clean, 0u, abort_flag))) {
+        if (!zb_mbar_wait(&v_full[stage], phase, abort_flag)) {
           *abort_where = 4u;
           break;
         }

@@ -408,14 +408,14 @@ def _prefill_short(hq: int, hd: int, seqs: int, longest: int) -> bool:
     7.3 / 8.6, 8.9 / 8.7; 8 and 32 of 128 with 16 9.0 / 8.8, 19.9 / 18.3; 20 of 100 with 16 / 32 13.3 / 14.8, 21.0 / 23.1; 64 of 64 with 4 / 16 / 32
     10.5 / 6.7, 17.9 / 21.1, 27.9 / 36.4.  head_dim 128: one of 1 / 128 with 32 5.7 / 6.9, 8.8 / 10.6, but 40 of 10 30.7 / 27.8.  head_dim
     256: never."""
-    if hd == 256 or longest > 128:
+    if longest > 128 or hd == 256:
         return False
     ctas, sms = seqs * hq // 2, _lib.lib().zb_num_sms()
     return ctas <= 32 or (hd == 64 and (ctas > 2 * sms or (ctas > sms and (longest <= 64 or 2 * ctas <= 3 * sms))))
 
 
 def prefill_on_tc(q, k_cache, ext=None) -> bool:
-    """Whether `paged_prefill` (impl "auto") runs the tcgen05 kernel."""
+    """Whether `paged_prefill` (impl "auto") runs a tcgen05 kernel; without `ext` short prompts may be faster on the other one."""
     return _ATTN_TC and _tc_takes(q, k_cache, ext)
 
 
@@ -440,14 +440,15 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
     assert q_start.dtype == torch.int32 and block_table.is_contiguous()
     if out is None:
         out = torch.empty((t, hq, hd), dtype=q.dtype, device=q.device)
-    if (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 or q.stride(0) % 8 or (ext is None and out.data_ptr() % 4):
+    at = out.data_ptr() if ext is None else 0
+    if (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 or q.stride(0) % 8 or at % 4:
         raise ValueError("prefill attention copies 16 bytes at a time: rows of q and the caches start on 16 bytes, those of out on 4")
     nqb = total_q_blocks if total_q_blocks is not None else t // 64 + b
     l = _lib.lib()
     scale = float(scale if scale is not None else 1.0 / math.sqrt(hd))
     # the tcgen05 kernel stores rows of 16-byte pieces and scales the row's maximum (no larger any more with a scale below zero) and the mask;
     # the other one stores 4 bytes at a time and takes the maximum of the scaled scores
-    tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or (out.data_ptr() % 16 == 0 and scale > 0))
+    tc_ok = _tc_takes(q, k_cache, ext) and (ext is not None or (at % 16 == 0 and scale > 0))
     if impl == "tc" and not tc_ok:
         raise ValueError(f"the tensor-core prefill kernel does not take hq={hq} hkv={hkv} hd={hd} page={page}")
     longest = max_seq_len if max_seq_len is not None else block_table.shape[1] * page
