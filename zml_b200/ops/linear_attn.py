@@ -99,12 +99,12 @@ def causal_conv1d(x, w, state, q_start, seq_lens, slots, pre=None, post=None, si
 def _delta_in_chunks(tokens: int, seqs: int, longest: Optional[int] = None) -> bool:
     """Whether a batch takes the chunked kernels (csrc/gated_delta_chunk.cu) instead of the walk token by token.  The walk takes 1.3 - 1.6 us
     a token of the longest sequence, the chunked kernels 19 us to begin with; with many sequences both are bound by the states they read and
-    write, 0.7 and 1.2 us a sequence.  32 heads of 128, us, chunked / walked: 1 sequence of 8 / 12 / 16 / 40 tokens 19 / 17, 19 / 23, 19 / 29,
+    write, 0.7 and 1.2 us a sequence.  An uneven batch goes by chunks where that gives more than the 10 us a layer that two more launches and a
+    workspace cost a host that is not ahead of the GPU (Qwen3.5, 16 layers, portions of 16, 9 and 3 tokens: 3033 us walked, 3144 by
+    chunks).  32 heads of 128, us, chunked / walked: 1 sequence of 8 / 12 / 16 / 40 tokens 19 / 17, 19 / 23, 19 / 29,
     23 / 67, of 4096 482 / 8179; 8 of 8 / 12 26 / 22, 28 / 30; 32 of 4 / 6 / 8 53 / 45, 53 / 61, 56 / 78; one of 200 beside 14 single tokens
     57 / 329, one of 16 / 24 / 40 beside 31 51 / 45, 53 / 59, 55 / 87, one of 32 / 64 beside 127 174 / 151, 178 / 215."""
-    if longest is None:
-        longest = tokens // max(1, seqs)
-    return longest > 10 + 0.31 * seqs or (seqs >= 16 and tokens >= 6 * seqs)
+    return tokens >= 16 * seqs or (seqs >= 16 and tokens >= 6 * seqs) or (longest is not None and longest > 16 + 0.3 * seqs)
 
 
 def _rows16(x) -> bool:
