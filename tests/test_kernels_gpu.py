@@ -464,6 +464,10 @@ def test_paged_prefill_alignment(hd):
             ops.paged_prefill(*args, bt, sl, qst)
     with pytest.raises(ValueError):
         ops.paged_prefill(q, kc, vc, bt, sl, qst, out=out, impl="tc")
+    one = torch.tensor([0, 1], dtype=torch.int32, device=DEV)
+    row = q[:1].as_strided((1, 4, hd), (4 * hd + 3, hd, 1))            # the stride of a single row says nothing about where rows start
+    want = ref.paged_attention(q[:1], kc, vc, bt[:1], [70], [0, 1])
+    expect_close(ops.paged_prefill(row, kc, vc, bt[:1], sl[:1], one).float(), want.float(), atol=2e-2, rtol=2e-2, min_close=ALL)
 
 
 @pytest.mark.parametrize("layout,rot", [(0, None), (1, None), (0, 32), (2, 32)])

@@ -441,7 +441,7 @@ def paged_prefill(q, k_cache, v_cache, block_table, seq_lens, q_start, scale: fl
     if out is None:
         out = torch.empty((t, hq, hd), dtype=q.dtype, device=q.device)
     at = out.data_ptr() if ext is None else 0
-    if (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 or q.stride(0) % 8 or at % 4:
+    if (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 or (t > 1 and q.stride(0) % 8) or at % 4:
         raise ValueError("prefill attention copies 16 bytes at a time: rows of q and the caches start on 16 bytes, those of out on 4")
     nqb = total_q_blocks if total_q_blocks is not None else t // 64 + b
     l = _lib.lib()
